@@ -223,6 +223,21 @@ struct HBHost {
     }
 };
 
+// Dynamic shared memory a kernel may be launched with, raised to at least `bytes` on the current
+// device and never lowered: the limit belongs to the function, and every handle of the process
+// launches with the size of its own system.
+void allow_smem(const void* kernel, size_t bytes)
+{
+    static std::mutex mu;
+    static std::map<std::pair<int, const void*>, size_t> limit;
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    size_t& l = limit[{dev, kernel}];
+    l = std::max(l, bytes);
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l));
+}
+
 // blocks of a tiled pair kernel: enough partner slices to give every SM a few blocks
 int pair_splits(int n, int max_range)
 {
@@ -1285,8 +1300,7 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
                 P.refine.alloc(1);
                 P.batch_smem = std::max<size_t>(P.batch_smem, (size_t)kTcSmemBytes);
             }
-            CK(cudaFuncSetAttribute((const void*)k_eeq_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)P.batch_smem));
+            allow_smem((const void*)k_eeq_batch, P.batch_smem);
             int per_sm = 0, nsm = 0;
             CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_eeq_batch, 512, P.batch_smem));
             CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, P.opt.device));
@@ -1488,7 +1502,7 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
             P.rdiag.alloc(P.nred);
             P.ysol.alloc(P.nred);
             P.chol_smem = (2 * CB * CLD + CB) * sizeof(double);
-            CK(cudaFuncSetAttribute((const void*)k_chol, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.chol_smem));
+            allow_smem((const void*)k_chol, P.chol_smem);
             int per_sm = 0;
             CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_chol, kCholThreads, P.chol_smem));
             P.chol_grid = std::max(1, std::min(per_sm * nsm, P.chol_ntasks));
@@ -1670,7 +1684,7 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
                 CK(cudaMemset(P.piters.p, 0, 2 * sizeof(int)));
                 P.pcg_grid = G;
                 P.pcg_smem = smem;
-                CK(cudaFuncSetAttribute((const void*)k_pcg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                allow_smem((const void*)k_pcg, smem);
                 int per_sm = 0;
                 CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_pcg, kPcgThreads, smem));
                 P.pcg_ready = per_sm >= 1;
@@ -1682,7 +1696,7 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
                     int ps = 0;
                     const void* kir = (const void*)k_pcg_ir;
                     if (P.pcg_smem_ir <= 220 * 1024) {
-                        CK(cudaFuncSetAttribute(kir, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.pcg_smem_ir));
+                        allow_smem(kir, P.pcg_smem_ir);
                         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, kir, kPcgThreads, P.pcg_smem_ir));
                     }
                     P.pcg_ir = ps >= 1;
@@ -1713,8 +1727,7 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
                                 P.pcg_res_ntl <= 5 && P.pcg_smem_res <= 200 * 1024;
                     if (P.pcg_res) {
                         P.prtiles.upload(rt);
-                        CK(cudaFuncSetAttribute((const void*)k_pcg_res, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int)P.pcg_smem_res));
+                        allow_smem((const void*)k_pcg_res, P.pcg_smem_res);
                         int rs = 0;
                         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rs, (const void*)k_pcg_res, kPcgPipeThreads,
                                                                          P.pcg_smem_res));
@@ -1722,8 +1735,7 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
                     }
                 }
                 if (P.pcg_pipe) {
-                    CK(cudaFuncSetAttribute((const void*)k_pcg_pipe, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)P.pcg_smem_pipe));
+                    allow_smem((const void*)k_pcg_pipe, P.pcg_smem_pipe);
                     int ps = 0;
                     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, (const void*)k_pcg_pipe, kPcgPipeThreads,
                                                                      P.pcg_smem_pipe));
