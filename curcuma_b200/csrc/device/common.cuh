@@ -125,6 +125,43 @@ __device__ __forceinline__ void block_add(double v, double* dst)
     }
 }
 
+// ---- asynchronous copies into shared memory (mbarriers; every wait is bounded) ----
+constexpr long long kTmaPolls = 1ll << 24;
+__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes)
+                 : "memory");
+}
+// true once the phase with the given parity has completed; false after kTmaPolls polls
+__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity)
+{
+    for (long long k = 0; k < kTmaPolls; ++k) {
+        unsigned done;
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                     " selp.u32 %0, 1, 0, p;\n}\n"
+                     : "=r"(done)
+                     : "r"(smem_u32(bar)), "r"(parity)
+                     : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
+// bytes (a multiple of 16, both addresses 16-byte aligned) of global memory into shared memory,
+// completing on bar
+__device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned bytes, unsigned long long* bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
+                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+
 // bond-angle cosine and d(theta)/dx (forcefieldfunctions.h:47-83)
 __device__ double angle_cos(D3 i, D3 j, D3 k, D3 d[3])
 {
@@ -239,6 +276,7 @@ struct View {
     const int2* jr;           // [first, last+1) atom range of the atom's molecule
     const int* perm;          // internal -> caller index
     const double4* pos;       // current geometry (bohr)
+    const double* msd;        // [2]: largest coordinate change since the set-up geometry
     const double4* pos0;      // setup geometry (bohr)
     const double* rcov_cn;
     const double* rcov43;     // 4/3 * covalent_rad_d3 (angle/torsion damping)
@@ -252,19 +290,29 @@ struct View {
     const int* slot;
     const int* nref;
     const double* refcn;      // n*7
-    const double* w0;         // n*7 setup weights
-    const double* g0;         // n*K*7 setup half contraction
-    const double* c6ref;      // K*K*49
+    // D4 reference data, packed: the references of the K elements present follow one another
+    // (element slot s from kofs[s], at most 7 each), Rp of them rounded up to a multiple of 4
+    // with zeros; an atom's row of weights is zero outside its own element.  zeta of the atom
+    // is folded into w0p, wp (and so into the partner's dot products), g0p and hdgp.  The rows
+    // are stored as matrix operands: 8 atoms x 4 references are 32 contiguous doubles (element
+    // (i, k) at pk(i, k)), so that a warp's operand load is one contiguous run; every molecule
+    // takes whole blocks of 32 rows (pshift added to its atom indexes), the gaps are zero.
+    int Rp;
+    const int* pshift;        // per molecule
+    const int* kof;           // first packed reference of each atom's element
+    const double* w0p;        // n*Rp setup weights
+    const double* g0p;        // n*Rp setup half contraction with every reference
+    const double* c6p;        // K*7*Rp reference C6: (slot, own reference, packed reference)
     const double* zeta;
     const double* szr;        // sqrt(0.5 r4/r2 sqrt Z)
+    const double* c4;         // (3 szr^2)^(1/4): the product of two is sqrt(r4r2) of the pair
+    const double* hmax;       // 72 max alpeeq: beyond this r^2 every Coulomb pair is 1/r
     // per step
     double* cnraw;
     double* cn;
     double* dlog;
-    double* w;                // n*7
-    double* dw;
-    double* hg;               // n*K*7
-    double* hdg;
+    double* wp;               // n*Rp current weights
+    double* hdgp;             // n*Rp half contraction of the weights' CN derivative
     double* q;
     double* dEdcn;
     double* v;
@@ -287,6 +335,12 @@ struct View {
     // take the minimum image; torsions, inversions, ATM, BATM and the EEQ matrix do not
     Cell cell;
 };
+
+// element (row, k) of a packed array (View), row = atom + pshift of its molecule
+__device__ __forceinline__ size_t pk(int Rp, int row, int k)
+{
+    return ((size_t)(row >> 3) * (Rp >> 2) + (k >> 2)) * 32 + (row & 7) * 4 + (k & 3);
+}
 
 // minimum-image difference pos[b] - pos[a] in FP64 (the plain difference without a cell)
 __device__ __forceinline__ D3 dmic(const View& V, int a, int b)

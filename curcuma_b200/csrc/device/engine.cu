@@ -51,6 +51,7 @@ namespace gfnff {
 #include "common.cuh"
 #include "k_bonded.cuh"
 #include "k_nonbonded.cuh"
+#include "k_pairs.cuh"
 #include "k_alpb.cuh"
 #include "k_eeq.cuh"
 #include "k_eeq_tc.cuh"
@@ -294,7 +295,8 @@ struct Engine::Impl {
     int n = 0, nfrag = 0, K = 0, nred = 0, nmol = 0, nsplit = 1;
     // Coulomb + D4 pairs: each pair once over a tile-pair list (default), or both
     // directions by rows (GFNFF_PAIRS=rows)
-    DBuf<int2> symtiles;
+    DBuf<int4> coul_tiles[3], d4_tiles[3];   // tile lists of k_pairs_coul and k_pairs_d4 per variant
+    int n_coul_tiles[3] = {0, 0, 0}, n_d4_tiles[3] = {0, 0, 0};
     DBuf<double4> boxlo, boxhi;   // per run of kBoxAtoms atoms
     // CN neighbour list (k_cn_nl, k_cn_chain_nl): pairs within 6 + kCnSkin bohr of the
     // reference geometry cnl_ref, CSR by atom; cnl_bad = 1 once an atom moved more than
@@ -383,16 +385,15 @@ struct Engine::Impl {
     }
     bool box_cull = false;        // CN kernels skip far tiles (single molecules >= 8192 atoms)
     Cell cell{};                  // periodic cell (cell.on = 0: isolated system)
-    int nsym = 0;
     bool pairs_sym = true;
-    bool pairs_occ = false;   // 10 blocks per SM (96 registers) instead of the unbounded 116
-    int pair_tile = 64;       // tile edge of k_pairs_sym
-    // Coulomb + D4 pair kernel variant, chosen at set-up by timing (tune_pairs): tile edge
-    // (atoms per block side) and blocks per SM of k_pairs_sym, or both directions by rows
+    bool pairs_occ = false;   // GFNFF_PAIRS_OCC=1: the untuned choice of single molecules is the largest tile
+    // Coulomb + D4 pair kernel variant, chosen at set-up by timing (tune_pairs): the tiles of
+    // k_pairs_coul and k_pairs_d4, or both directions by rows (k_pairs).  Small tiles give small
+    // systems enough warps; large ones add their partner sums to memory once per 128 rows.  The
+    // D4 tiles are one warp high, so that a warp whose rows are out of range does not wait.
     enum { PAIRS_SYM32 = 0, PAIRS_SYM64 = 1, PAIRS_SYM64_OCC = 2, PAIRS_ROWS = 3 };
+    static constexpr int kCoulRows[3] = {32, 64, 128}, kD4Rows[3] = {32, 32, 32}, kPairCols[3] = {16, 32, 64};
     int pair_variant = PAIRS_SYM64;
-    DBuf<int2> symtiles32;    // tile list of the 32-atom variant (symtiles: 64)
-    int nsym32 = 0;
     float pair_ms[4] = {-1.f, -1.f, -1.f, -1.f};   // the tuner's timings (ms per launch)
     // D4 pairs (charge-independent) on the side stream beside the EEQ solve, Coulomb pairs
     // after it on the main stream (GFNFF_PAIRS_SPLIT=0: both in one pass after the solve)
@@ -405,8 +406,12 @@ struct Engine::Impl {
     DBuf<double> e0;
     // model
     DBuf<double4> pos, pos0, hbref, toporef;
-    DBuf<double> rcov_cn, rcov43, rcov_d3, chi_base, cnf, gam, alpeeq, adiag, qa, refcn, w0, g0, c6ref, zeta, szr;
+    DBuf<double> rcov_cn, rcov43, rcov_d3, chi_base, cnf, gam, alpeeq, adiag, qa, refcn, zeta, szr;
     DBuf<int> slot, nref;
+    // packed D4 reference data (View)
+    int Rp = 0;
+    DBuf<int> kof, pshift;
+    DBuf<double> w0p, g0p, c6p, c4, hmax;
     // EEQ structure
     DBuf<int> red2atom, atom2red, anchor, frag_off, frag_atoms, qlist, roff;
     DBuf<long long> moff;
@@ -547,7 +552,7 @@ struct Engine::Impl {
     DBuf<double> r_al, r_ab;
     DBuf<unsigned char> r_kind;
     // per step
-    DBuf<double> cnraw, cn, dlog, w, dw, hg, hdg, q, dEdcn, v, grad, E, M, bvec, xyz_stage, msd;
+    DBuf<double> cnraw, cn, dlog, wp, hdgp, q, dEdcn, v, grad, E, M, bvec, xyz_stage, msd;
     DBuf<double> gout, qout, cnout;
     DBuf<double> work;
     DBuf<int> info, info2, status, ipiv, bad;
@@ -691,16 +696,28 @@ struct Engine::Impl {
         if (graph) cudaGraphExecDestroy(graph);
         graph = nullptr;
     }
-    // one launch of the chosen Coulomb + D4 pair kernel variant (PART: the terms)
+    // one launch of the chosen Coulomb or D4 pair kernel variant (PART: the term)
+    template <int PART, int WR, int COLS>
+    void launch_pairs_tile(const View& V, const int4* tl, int nt, cudaStream_t st)
+    {
+        if constexpr (PART == kPairD4) {
+            if (V.cell.on) k_pairs_d4<WR, COLS, true><<<nt, 32 * WR, 0, st>>>(V, tl);
+            else k_pairs_d4<WR, COLS, false><<<nt, 32 * WR, 0, st>>>(V, tl);
+        } else {
+            if (V.cell.on) k_pairs_coul<WR, COLS, true, false><<<nt, 32 * WR, 0, st>>>(V, tl);   // exact mode refuses a cell
+            else if (V.cfar) k_pairs_coul<WR, COLS, false, true><<<nt, 32 * WR, 0, st>>>(V, tl);
+            else k_pairs_coul<WR, COLS, false, false><<<nt, 32 * WR, 0, st>>>(V, tl);
+        }
+    }
     template <int PART>
     void launch_pairs_sym(int variant, const View& V, cudaStream_t st)
     {
-        if (variant == PAIRS_SYM32)
-            k_pairs_sym<double, 16, 32, PART><<<nsym32, 32, 0, st>>>(V, symtiles32.p);
-        else if (variant == PAIRS_SYM64_OCC)
-            k_pairs_sym<double, 10, kST, PART><<<nsym, kST, 0, st>>>(V, symtiles.p);
-        else
-            k_pairs_sym<double, 8, kST, PART><<<nsym, kST, 0, st>>>(V, symtiles.p);
+        constexpr bool D4 = PART == kPairD4;
+        const int4* tl = (D4 ? d4_tiles : coul_tiles)[variant].p;
+        const int nt = (D4 ? n_d4_tiles : n_coul_tiles)[variant];
+        if (variant == PAIRS_SYM32) launch_pairs_tile<PART, 1, 16>(V, tl, nt, st);
+        else if (variant == PAIRS_SYM64) launch_pairs_tile<PART, D4 ? 1 : 2, 32>(V, tl, nt, st);
+        else launch_pairs_tile<PART, D4 ? 1 : 4, 64>(V, tl, nt, st);
     }
     cudaEvent_t ev[Engine::kNumPhases + 1] = {};
     void mark(int k)
@@ -717,9 +734,10 @@ struct Engine::Impl {
         V.mol = mol.p; V.jr = jr.p; V.perm = perm.p;
         V.pos = pos.p; V.pos0 = pos0.p; V.rcov_cn = rcov_cn.p; V.rcov43 = rcov43.p; V.rcov_d3 = rcov_d3.p;
         V.chi_base = chi_base.p; V.cnf = cnf.p; V.gam = gam.p; V.alpeeq = alpeeq.p; V.adiag = adiag.p; V.qa = qa.p;
-        V.slot = slot.p; V.nref = nref.p; V.refcn = refcn.p; V.w0 = w0.p; V.g0 = g0.p; V.c6ref = c6ref.p;
-        V.zeta = zeta.p; V.szr = szr.p;
-        V.cnraw = cnraw.p; V.cn = cn.p; V.dlog = dlog.p; V.w = w.p; V.dw = dw.p; V.hg = hg.p; V.hdg = hdg.p;
+        V.slot = slot.p; V.nref = nref.p; V.refcn = refcn.p;
+        V.Rp = Rp; V.kof = kof.p; V.pshift = pshift.p; V.w0p = w0p.p; V.g0p = g0p.p; V.c6p = c6p.p;
+        V.zeta = zeta.p; V.szr = szr.p; V.c4 = c4.p; V.hmax = hmax.p; V.msd = msd.p;
+        V.cnraw = cnraw.p; V.cn = cn.p; V.dlog = dlog.p; V.wp = wp.p; V.hdgp = hdgp.p;
         V.q = q.p; V.dEdcn = dEdcn.p; V.v = v.p; V.grad = grad.p; V.E = E.p; V.status = status.p;
         V.brad = alpb_on ? ab.brad.p : nullptr;
         V.bdiag = alpb_on ? ab.bdiag.p : nullptr;
@@ -1061,35 +1079,38 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
     int max_range = 0;
     for (int m = 0; m < nm; ++m) max_range = std::max(max_range, mols[m]->n);
     P.nsplit = pair_splits(n, max_range);
-    {   // tile pairs (i tile <= j tile, both within the tile's molecules) of k_pairs_sym
-        // both tile edges (the tuner picks one): tile pairs I <= J within the rows' molecules
-        auto tiles = [&](int T) {
-            std::vector<int2> tl;
-            const int nt = (n + T - 1) / T;
-            for (int I = 0; I < nt; ++I) {
-                const int i0 = I * T, hi = hjr[std::min(n, i0 + T) - 1].y;
-                for (int J = I; J * T < hi; ++J) tl.push_back(make_int2(i0, J * T));
-            }
+    {   // tiles of k_pairs_coul / k_pairs_d4 per molecule: row blocks from the molecule's first atom, their
+        // partners from the block's first row on; by increasing distance from the diagonal, so
+        // that the costlier near tiles (erf, exp, D4) start first
+        auto tiles = [&](int TR, int TC) {
+            std::vector<int4> tl;
+            for (int d = 0; d < max_range; d += TC)
+                for (int m = 0; m < nm; ++m) {
+                    const int a0 = P.h_aoff[m], a1 = P.h_aoff[m + 1];
+                    for (int i0 = a0; i0 + d < a1; i0 += TR)
+                        tl.push_back(make_int4(i0, std::min(i0 + TR, a1), i0 + d, std::min(i0 + d + TC, a1)));
+                }
             return tl;
         };
-        const std::vector<int2> tl = tiles(kST), tl32 = tiles(32);
-        P.symtiles.upload(tl);
-        P.symtiles32.upload(tl32);
-        P.nsym32 = (int)tl32.size();
-        P.pair_tile = nm > 1 ? 32 : kST;
+        for (int v = 0; v < 3; ++v) {
+            const std::vector<int4> c = tiles(Impl::kCoulRows[v], Impl::kPairCols[v]);
+            const std::vector<int4> d = tiles(Impl::kD4Rows[v], Impl::kPairCols[v]);
+            P.coul_tiles[v].upload(c);
+            P.d4_tiles[v].upload(d);
+            P.n_coul_tiles[v] = (int)c.size();
+            P.n_d4_tiles[v] = (int)d.size();
+        }
         P.boxlo.alloc((n + kBoxAtoms - 1) / kBoxAtoms);
         P.boxhi.alloc((n + kBoxAtoms - 1) / kBoxAtoms);
         // box tests compare plain coordinates: off in a periodic cell
         P.box_cull = nm == 1 && n >= 8192 && !P.cell.on;
-        P.nsym = (int)tl.size();
         const char* pe = std::getenv("GFNFF_PAIRS");
         P.pairs_sym = !(pe && !std::strcmp(pe, "rows"));
         const char* po = std::getenv("GFNFF_PAIRS_OCC");
         P.pairs_occ = po && !std::strcmp(po, "1");
-        // the variant before tuning (batches: 32-atom tiles, which straddle fewer molecules)
+        // the variant before tuning
         P.pair_variant = !P.pairs_sym ? Impl::PAIRS_ROWS
-                         : (P.pair_tile == 32 ? Impl::PAIRS_SYM32
-                                              : (P.pairs_occ ? Impl::PAIRS_SYM64_OCC : Impl::PAIRS_SYM64));
+                         : (nm > 1 ? Impl::PAIRS_SYM32 : (P.pairs_occ ? Impl::PAIRS_SYM64_OCC : Impl::PAIRS_SYM64));
         const char* ps = std::getenv("GFNFF_PAIRS_SPLIT");
         P.pairs_split = !ps ? 1 : (!std::strcmp(ps, "0") ? 0 : (!std::strcmp(ps, "1") ? 2 : 1));
     }
@@ -1122,8 +1143,33 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
     // ---- per-atom data in internal order ----
     std::vector<double4> p0(n);
     std::vector<double> rcn(n), r43(n), rd3(n), chi(n), cnf(n), gam(n), alp(n), adg(n), qa(n), zeta(n), szr(n);
-    std::vector<double> rcn7((size_t)n * 7), w07((size_t)n * 7), g0((size_t)n * K * 7, 0.0);
+    std::vector<double> rcn7((size_t)n * 7), c4(n);
     std::vector<int> slot(n), nref(n);
+    // packed references: the most that an atom of each element has, in slot order
+    std::vector<int> kofs(K + 1, 0);
+    for (int m = 0; m < nm; ++m)
+        for (int a = 0; a < mols[m]->n; ++a) {
+            int& c = kofs[gslot[m][mols[m]->slot[a]] + 1];
+            c = std::max(c, mols[m]->nref[a]);
+        }
+    for (int t = 0; t < K; ++t) kofs[t + 1] += kofs[t];
+    const int Rp = std::max(4, (kofs[K] + 3) & ~3);
+    P.Rp = Rp;
+    std::vector<int> pshift(nm);
+    int prows = 0;   // packed rows: every molecule takes whole blocks of 32 (a warp's rows)
+    for (int m = 0; m < nm; ++m) {
+        pshift[m] = prows - P.h_aoff[m];
+        prows = (prows + mols[m]->n + 31) & ~31;
+    }
+    if ((long long)prows * Rp > std::numeric_limits<int>::max()) throw std::runtime_error("too many atoms for the packed D4 rows");
+    auto pkh = [Rp](int row, int k) { return ((size_t)(row >> 3) * (Rp >> 2) + (k >> 2)) * 32 + (row & 7) * 4 + (k & 3); };
+    std::vector<double> w0p((size_t)prows * Rp, 0.0), g0p((size_t)prows * Rp, 0.0), c6p((size_t)K * 7 * Rp, 0.0);
+    std::vector<int> kof(n);
+    for (int s = 0; s < K; ++s)
+        for (int a = 0; a < 7; ++a)
+            for (int t = 0; t < K; ++t)
+                for (int b = 0; b < kofs[t + 1] - kofs[t]; ++b)
+                    c6p[((size_t)s * 7 + a) * Rp + kofs[t] + b] = c6g[((size_t)s * K + t) * 49 + a * 7 + b];
     std::vector<double> e0(nm);
     for (int m = 0; m < nm; ++m) {
         const Model& M = *mols[m];
@@ -1136,15 +1182,16 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
             adg[s] = M.gam[a] + 0.797884560802866 / std::sqrt(M.alpeeq[a]);
             qa[s] = M.qa[a]; zeta[s] = M.zeta[a]; szr[s] = M.sqrt_zr4r2[a];
             slot[s] = gslot[m][M.slot[a]]; nref[s] = M.nref[a];
-            for (int r = 0; r < 7; ++r) { rcn7[(size_t)s * 7 + r] = M.refcn[(size_t)a * 7 + r]; w07[(size_t)s * 7 + r] = M.w_setup[(size_t)a * 7 + r]; }
+            for (int r = 0; r < 7; ++r) rcn7[(size_t)s * 7 + r] = M.refcn[(size_t)a * 7 + r];
+            kof[s] = kofs[slot[s]];
+            c4[s] = std::sqrt(std::sqrt(3.0) * szr[s]);
             // frozen half contraction at the setup weights (d4param_generator.cpp:1235-1290)
-            for (int t = 0; t < K; ++t) {
-                const double* C = &c6g[(((size_t)slot[s] * K + t) * 7) * 7];
-                for (int b = 0; b < 7; ++b) {
-                    double v = 0.0;
-                    for (int r = 0; r < nref[s]; ++r) v += w07[(size_t)s * 7 + r] * C[r * 7 + b];
-                    g0[((size_t)s * K + t) * 7 + b] = v;
-                }
+            const double* w = &M.w_setup[(size_t)a * 7];
+            for (int r = 0; r < nref[s]; ++r) w0p[pkh(s + pshift[m], kof[s] + r)] = zeta[s] * w[r];
+            for (int k = 0; k < Rp; ++k) {
+                double v = 0.0;
+                for (int r = 0; r < nref[s]; ++r) v += w[r] * c6p[((size_t)slot[s] * 7 + r) * Rp + k];
+                g0p[pkh(s + pshift[m], k)] = zeta[s] * v;
             }
         }
     }
@@ -1163,8 +1210,10 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
     }
     P.rcov_cn.upload(rcn); P.rcov43.upload(r43); P.rcov_d3.upload(rd3);
     P.chi_base.upload(chi); P.cnf.upload(cnf); P.gam.upload(gam); P.alpeeq.upload(alp); P.adiag.upload(adg);
-    P.qa.upload(qa); P.slot.upload(slot); P.nref.upload(nref); P.refcn.upload(rcn7); P.w0.upload(w07);
-    P.c6ref.upload(c6g); P.zeta.upload(zeta); P.szr.upload(szr); P.g0.upload(g0); P.e0.upload(e0);
+    P.qa.upload(qa); P.slot.upload(slot); P.nref.upload(nref); P.refcn.upload(rcn7);
+    P.kof.upload(kof); P.pshift.upload(pshift); P.w0p.upload(w0p); P.g0p.upload(g0p); P.c6p.upload(c6p); P.c4.upload(c4);
+    P.hmax.upload({72.0 * *std::max_element(alp.begin(), alp.end())});
+    P.zeta.upload(zeta); P.szr.upload(szr); P.e0.upload(e0);
     // ---- EEQ null-space structure (global fragment ids, reduced index per molecule) ----
     {
         std::vector<int> fragi(n);
@@ -1448,8 +1497,9 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
         P.x_a.upload(xa); P.x_x.upload(xx); P.x_b.upload(xb); P.x_pre.upload(xpre); P.x_rv.upload(xrv);
     }
     // ---- per-step buffers ----
-    P.cnraw.alloc(n); P.cn.alloc(n); P.dlog.alloc(n); P.w.alloc((size_t)n * 7); P.dw.alloc((size_t)n * 7);
-    P.hg.alloc((size_t)n * K * 7); P.hdg.alloc((size_t)n * K * 7);
+    P.cnraw.alloc(n); P.cn.alloc(n); P.dlog.alloc(n); 
+    P.wp.upload(std::vector<double>((size_t)prows * Rp, 0.0));     // zero outside each atom's element
+    P.hdgp.upload(std::vector<double>((size_t)prows * Rp, 0.0));   // and in the gaps between molecules
     P.etot.alloc(nm);
     {   // charge response only where a pair can exceed the 100 bohr Coulomb cut
         double ext = 0.0;
@@ -1470,7 +1520,7 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
     P.gout.alloc(3 * (size_t)n); P.qout.alloc(n); P.cnout.alloc(n);
     P.lda = (P.nred + 4) & ~3;   // >= nred + 1, a multiple of 4: 16-byte aligned FP32 and FP64 columns
     P.M.alloc((size_t)std::max<long long>(1, nm == 1 ? (long long)P.lda * P.nred : P.msize));
-    P.bvec.alloc(std::max(1, P.nred)); P.xyz_stage.alloc(3 * (size_t)n); P.msd.alloc(2);
+    P.bvec.alloc(std::max(1, P.nred)); P.xyz_stage.alloc(3 * (size_t)n); P.msd.alloc(3);
     P.info.alloc(nm); P.info2.alloc(1); P.status.alloc(nm); P.bad.alloc(nm);
     CK(cudaMemset(P.info.p, 0, nm * sizeof(int)));
     P.use_lu = false;
@@ -1824,13 +1874,13 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
     P.pcg_warm = !(warm_env && !std::strcmp(warm_env, "0"));
 }
 
-// Tile-shape autotuner of the Coulomb + D4 pair kernel.  Candidates: k_pairs_sym with 32- or
-// 64-atom tiles (a block is one warp or two; the tile edge is the atom block width and the
-// partners a warp takes per step), the 64-atom tiles also at 10 blocks per SM (96 registers)
-// instead of 8, and both directions by rows (k_pairs).  After one evaluation at the set-up
-// geometry (valid charges and weights in the buffers), each candidate runs once untimed and
-// three times between CUDA events on the handle's stream (both terms, PART = both); the
-// fastest is kept.  The pick is cached per (device, batch or single molecule, size bucket
+// Tile-shape autotuner of the Coulomb and D4 pair kernels.  Candidates: k_pairs_coul / k_pairs_d4
+// with tiles of 32 x 16 (rows x partners), 64 x 32 / 32 x 32 and 128 x 64 / 32 x 64 atoms, and
+// both directions by rows (k_pairs).  After one evaluation at the set-up geometry (valid charges
+// and weights in the buffers), each candidate runs once untimed and three times between CUDA
+// events on the handle's stream (both terms); the fastest is kept.  32 x 16 wins up to ~4000 atoms
+// (194 atoms 27 against 58 us for 128 x 64, 1000 waters 72 / 93 us), 128 x 64 on 20,480 atoms
+// (1.36 against 1.72 ms).  The pick is cached per (device, batch or single molecule, size bucket
 // floor(log2 N)) for the process, so further handles of similar systems skip the timing.
 // GFNFF_PAIRS_TUNE=0, GFNFF_PAIRS=rows and GFNFF_PAIRS_OCC=1 keep the untuned choice;
 // GFNFF_PAIRS_VARIANT=sym32|sym64|sym64_occ10|rows forces one.
@@ -1878,8 +1928,11 @@ void Engine::tune_pairs(const std::vector<const Model*>& mols)
     int pick = P.pair_variant;
     for (int v = 0; v < 4; ++v) {
         auto run = [&]() {
-            if (v == Impl::PAIRS_ROWS) k_pairs<double><<<tgrid, kTile, 0, P.stream>>>(V, P.nsplit);
-            else P.launch_pairs_sym<kPairBoth>(v, V, P.stream);
+            if (v == Impl::PAIRS_ROWS) k_pairs<<<tgrid, kTile, 0, P.stream>>>(V, P.nsplit);
+            else {
+                P.launch_pairs_sym<kPairD4>(v, V, P.stream);
+                P.launch_pairs_sym<kPairCoul>(v, V, P.stream);
+            }
         };
         run();
         CK(cudaEventRecord(e0, P.stream));
@@ -2050,10 +2103,10 @@ void Engine::launch_positions(const double* d_xyz, bool bohr)
 {
     Impl& P = *p_;
     P.mark(0);
-    CK(cudaMemsetAsync(P.msd.p, 0, 2 * sizeof(double), P.stream));
+    CK(cudaMemsetAsync(P.msd.p, 0, 3 * sizeof(double), P.stream));
     k_positions<<<nblk(P.n), kBlock, 0, P.stream>>>(P.n, P.perm.p, d_xyz, bohr ? 1.0 : kAngToBohr, P.pos.p,
                                                    P.hbref.p, P.msd.p, P.cnl_on ? P.cnl_ref.p : nullptr,
-                                                   0.25 * Impl::kCnSkin * Impl::kCnSkin, P.cnl_bad.p, P.toporef.p);
+                                                   0.25 * Impl::kCnSkin * Impl::kCnSkin, P.cnl_bad.p, P.toporef.p, P.pos0.p);
 }
 
 // everything after the positions, reading and writing engine buffers only, so that it
@@ -2159,7 +2212,7 @@ void Engine::launch_body()
         (mixed ? k_cn<float> : k_cn<double>)<<<tgrid, kTile, 0, s>>>(V, P.nsplit, nullptr);
     }
     P.mark(2);
-    k_d4_weights<<<nblk(n), kBlock, 0, s>>>(V);
+    k_d4_weights<<<nblk((long)n * 8), kBlock, 0, s>>>(V);
     if (early) {
         CK(cudaEventRecord(P.ev_fork1, s));
         CK(cudaStreamWaitEvent(s2, P.ev_fork1, 0));
@@ -2236,9 +2289,10 @@ void Engine::launch_body()
         P.mark(7);
         hb_rep_terms();
     }
-    if (split) pairs_sym(std::integral_constant<int, kPairCoul>{}, s);
-    else if (P.pairs_sym) pairs_sym(std::integral_constant<int, kPairBoth>{}, s);
-    else k_pairs<double><<<tgrid, kTile, 0, s>>>(V, P.nsplit);
+    if (P.pairs_sym) {
+        if (!split) pairs_sym(std::integral_constant<int, kPairD4>{}, s);
+        pairs_sym(std::integral_constant<int, kPairCoul>{}, s);
+    } else k_pairs<<<tgrid, kTile, 0, s>>>(V, P.nsplit);
     if (P.resp_on) {
         // u = B M^-1 B^T w with the factor (or the iteration) of this step's EEQ matrix
         k_resp_rhs<<<nblk(P.nred), kBlock, 0, s>>>(V, P.red2atom.p, P.anchor.p, P.bres.p);
@@ -2384,6 +2438,8 @@ void Engine::update_eeq_parameters(const Model& m)
     CK(cudaMemcpy(P.cnf.p, cnf.data(), b, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(P.gam.p, gam.data(), b, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(P.alpeeq.p, alp.data(), b, cudaMemcpyHostToDevice));
+    const double hm = 72.0 * *std::max_element(alp.begin(), alp.end());
+    CK(cudaMemcpy(P.hmax.p, &hm, sizeof(hm), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(P.adiag.p, adg.data(), b, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(P.qa.p, qa.data(), b, cudaMemcpyHostToDevice));
     P.hbd.topo = nullptr;   // the HB detection's topology inputs follow the new topology

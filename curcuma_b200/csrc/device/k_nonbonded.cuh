@@ -34,18 +34,21 @@ __device__ __forceinline__ void tile_range(const View& V, int i0, int nsplit, in
 // sqrt(nl_lim2) away from it marks the list stale (kept until the host rebuilds it).
 // msd[1] receives the topology refresh metric, the largest |coordinate change| since the
 // geometry topo_ref of the last topology (gfnff_method.cpp:1021-1031), as the bits of a
-// non-negative double (which order like the integers)
+// non-negative double (which order like the integers); msd[2] the largest |coordinate change|
+// since the set-up geometry pos0 (all atoms of a batch)
 __global__ void k_positions(int n, const int* __restrict__ perm, const double* __restrict__ xyz, double scale,
                             double4* pos, const double4* __restrict__ ref, double* msd,
                             const double4* __restrict__ nl_ref, double nl_lim2, int* nl_bad,
-                            const double4* __restrict__ topo_ref)
+                            const double4* __restrict__ topo_ref, const double4* __restrict__ pos0)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double s = 0.0, dmax = 0.0;
+    double s = 0.0, dmax = 0.0, d0max = 0.0;
     if (i < n) {
         const int o = perm[i];
         const double x = xyz[3 * o] * scale, y = xyz[3 * o + 1] * scale, z = xyz[3 * o + 2] * scale;
         pos[i] = make_double4(x, y, z, 0.0);
+        const double4 p0 = pos0[i];
+        d0max = fmax(fabs(x - p0.x), fmax(fabs(y - p0.y), fabs(z - p0.z)));
         const double4 r = ref[i];
         s = (x - r.x) * (x - r.x) + (y - r.y) * (y - r.y) + (z - r.z) * (z - r.z);
         const double4 t = topo_ref[i];
@@ -56,9 +59,16 @@ __global__ void k_positions(int n, const int* __restrict__ perm, const double* _
             if (d2 > nl_lim2) atomicOr(nl_bad, 1);
         }
     }
-    for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
-    if ((threadIdx.x & 31) == 0 && dmax > 0.0)
-        atomicMax(reinterpret_cast<unsigned long long*>(msd + 1), (unsigned long long)__double_as_longlong(dmax));
+    for (int o = 16; o > 0; o >>= 1) {
+        dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+        d0max = fmax(d0max, __shfl_xor_sync(0xffffffffu, d0max, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (dmax > 0.0)
+            atomicMax(reinterpret_cast<unsigned long long*>(msd + 1), (unsigned long long)__double_as_longlong(dmax));
+        if (d0max > 0.0)
+            atomicMax(reinterpret_cast<unsigned long long*>(msd + 2), (unsigned long long)__double_as_longlong(d0max));
+    }
     block_add(s, msd);
 }
 
@@ -188,53 +198,57 @@ __global__ void __launch_bounds__(kTile) k_cn(View V, int nsplit, const int* nl_
 // CN log-squash (cnmax = 4.4) and its derivative, D4 Gaussian weights (wf = 4) and the
 // half contraction with the reference C6 (d4param_generator.cpp:1079-1290, :1692-1740)
 // ------------------------------------------------------------------------------------
-__global__ void k_d4_weights(View V)
+// Eight lanes per atom: lane r holds reference r (7 at most), so the exponentials of an atom run
+// side by side, and the lanes then share the half contraction over the packed references (a
+// thread per atom took 14 us on 194 atoms and 24 us on 20,480: a chain of 7 exp and K 49 loads).
+__global__ void __launch_bounds__(kBlock) k_d4_weights(View V)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= V.n) return;
-    {
-        const double cnmax = 4.4, s = V.cnraw[i];
-        V.cn[i] = log(1.0 + exp(cnmax)) - log(1.0 + exp(cnmax - s));
-        V.dlog[i] = exp(cnmax) / (exp(cnmax) + exp(s));
-    }
+    constexpr unsigned full = 0xffffffffu;
+    const int i0 = (blockIdx.x * kBlock + threadIdx.x) >> 3, r = threadIdx.x & 7;
+    const int i = min(i0, V.n - 1);   // whole warps stay: the lanes exchange values
+    const double cnmax = 4.4, s = V.cnraw[i];
+    const double cn = log(1.0 + exp(cnmax)) - log(1.0 + exp(cnmax - s));
     const int nr = V.nref[i];
-    const double cn = V.cn[i];
-    double ex[7], dex[7], w[7], dw[7];
-    double norm = 0.0, dnorm = 0.0;
-    for (int r = 0; r < 7; ++r) {
-        ex[r] = dex[r] = w[r] = dw[r] = 0.0;
-        if (r < nr) {
-            const double d = cn - V.refcn[i * 7 + r];
-            ex[r] = exp(-4.0 * d * d);
-            dex[r] = (-2.0 * 4.0) * d * ex[r];
-            norm += ex[r];
-            dnorm += dex[r];
-        }
+    double ex = 0.0, dex = 0.0;
+    if (r < nr) {
+        const double d = cn - V.refcn[i * 7 + r];
+        ex = exp(-4.0 * d * d);
+        dex = (-2.0 * 4.0) * d * ex;
     }
-    if (nr > 0) {
+    double norm = ex, dnorm = dex;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+        norm += __shfl_xor_sync(full, norm, o);
+        dnorm += __shfl_xor_sync(full, dnorm, o);
+    }
+    double w = 0.0, dw = 0.0;
+    if (r < nr) {
         if (norm > 1e-10) {
             const double inv = 1.0 / norm, inv2 = 1.0 / (norm * norm);
-            for (int r = 0; r < nr; ++r) {
-                w[r] = ex[r] * inv;
-                dw[r] = (dex[r] * norm - ex[r] * dnorm) * inv2;
-            }
+            w = ex * inv;
+            dw = (dex * norm - ex * dnorm) * inv2;
         } else {
-            w[0] = 1.0;
+            w = r == 0 ? 1.0 : 0.0;
         }
     }
-    for (int r = 0; r < 7; ++r) { V.w[i * 7 + r] = w[r]; V.dw[i * 7 + r] = dw[r]; }
-    const int si = V.slot[i];
-    for (int s = 0; s < V.K; ++s) {
-        const double* C = V.c6ref + ((size_t)(si * V.K + s)) * 49;
-        for (int b = 0; b < 7; ++b) {
-            double g = 0.0, dg = 0.0;
-            for (int a = 0; a < nr; ++a) {
-                g += w[a] * C[a * 7 + b];
-                dg += dw[a] * C[a * 7 + b];
-            }
-            V.hg[((size_t)i * V.K + s) * 7 + b] = g;
-            V.hdg[((size_t)i * V.K + s) * 7 + b] = dg;
-        }
+    const double z = V.zeta[i];
+    const bool act = i0 < V.n;
+    if (act && r == 0) {
+        V.cn[i] = cn;
+        V.dlog[i] = exp(cnmax) / (exp(cnmax) + exp(s));
+    }
+    const int row = i + V.pshift[V.nmol == 1 ? 0 : V.mol[i]];
+    if (act && r < nr) V.wp[pk(V.Rp, row, V.kof[i] + r)] = z * w;
+    const double* C = V.c6p + (size_t)V.slot[i] * 7 * V.Rp;
+    double dwa[7];
+#pragma unroll
+    for (int a = 0; a < 7; ++a) dwa[a] = __shfl_sync(full, dw, (threadIdx.x & 24) + a);
+    for (int k = r; k < V.Rp; k += 8) {
+        double dg = 0.0;
+#pragma unroll
+        for (int a = 0; a < 7; ++a)
+            if (a < nr) dg += dwa[a] * C[a * V.Rp + k];
+        if (act) V.hdgp[pk(V.Rp, row, k)] = z * dg;
     }
 }
 
@@ -292,54 +306,49 @@ __global__ void __launch_bounds__(kBlock) k_repulsion(View V, const int* off, co
 // Coulomb fast path: erf(x) rounds to exactly 1 in double for x >= 6 (erfc(6) = 2.2e-17
 // is below half an ulp of 1), i.e. for r^2 >= 36 (a_i + a_j); the pair is then q q / r and
 // its exp(-x^2) gradient term is below 2e-15 relative, so both are dropped there.
-// R is the arithmetic type of the D4 part beyond 15 bohr: double in the FP64 form,
-// float in the mixed form (nearer D4 pairs are FP64 in both).  Coulomb (both branches), the distances and every sum stay FP64 in both forms:
-// single Coulomb pairs reach 0.1 Eh and there are ~N^2/2 of them, so FP32 rounding in
-// them would add up to more than 1e-6 Eh.
+// This kernel (each block a run of atoms against all partners, both directions of a pair) is the
+// plain form of the terms; k_pairs_coul and k_pairs_d4 (k_pairs.cuh) evaluate the same pairs once.  It is one of
+// the set-up tuner's variants ("rows").
 // ------------------------------------------------------------------------------------
-// one D4 pair in arithmetic type R: energy e, dE/dr / r in dedr, dE/dCN_i in dc
-template <class R>
-__device__ __forceinline__ void d4_pair(double d2, const double* g0, const double* dg, const double (*sw0)[kTile],
+// one D4 pair: energy e, dE/dr / r in dedr, dE/dCN_i in dc (zeta folded into the operands)
+__device__ __forceinline__ void d4_pair(const View& V, double d2, int rowi, int kj, const double (*sw0)[kTile],
                                         const double (*sw)[kTile], int jj, int nr, double szi, double szj,
-                                        double zz_d, double& e, double& dedr, double& dc)
+                                        double& e, double& dedr, double& dc)
 {
-    R c6 = R(0), dc6 = R(0);
+    double c6 = 0.0, dc6 = 0.0;
     for (int b = 0; b < nr; ++b) {
-        c6 += (R)__ldg(g0 + b) * (R)sw0[b][jj];
-        dc6 += (R)dg[b] * (R)sw[b][jj];
+        c6 += V.g0p[pk(V.Rp, rowi, kj + b)] * sw0[b][jj];
+        dc6 += V.hdgp[pk(V.Rp, rowi, kj + b)] * sw[b][jj];
     }
-    const R q2 = (R)d2;
-    const R r4r2 = R(3) * (R)szi * (R)szj;
-    const R t = R(0.58) * sqrt(r4r2) + R(4.80);
-    const R r0sq = t * t;
-    const R zz = (R)zz_d;
-    const R r6 = q2 * q2 * q2, r06 = r0sq * r0sq * r0sq;
-    const R t6 = R(1) / (r6 + r06);
-    const R t8 = R(1) / (r6 * q2 + r06 * r0sq);
-    const R sum = t6 + R(2) * r4r2 * t8;
-    e = -(double)(c6 * sum * zz);
-    const R d6 = R(-6) * q2 * q2 * t6 * t6, d8 = R(-8) * r6 * t8 * t8;
-    dedr = -(double)(c6 * zz * (d6 + R(2) * r4r2 * d8));
-    dc = -(double)(dc6 * sum * zz);
+    const double q2 = d2;
+    const double r4r2 = 3.0 * szi * szj;
+    const double t = 0.58 * sqrt(r4r2) + 4.80;
+    const double r0sq = t * t;
+    const double r6 = q2 * q2 * q2, r06 = r0sq * r0sq * r0sq;
+    const double t6 = 1.0 / (r6 + r06);
+    const double t8 = 1.0 / (r6 * q2 + r06 * r0sq);
+    const double sum = t6 + 2.0 * r4r2 * t8;
+    e = -(c6 * sum);
+    const double d6 = -6.0 * q2 * q2 * t6 * t6, d8 = -8.0 * r6 * t8 * t8;
+    dedr = -(c6 * (d6 + 2.0 * r4r2 * d8));
+    dc = -(dc6 * sum);
 }
 
-template <class R>
 __global__ void __launch_bounds__(kTile) k_pairs(View V, int nsplit)
 {
     __shared__ double sx[kTile], sy[kTile], sz[kTile], s0x[kTile], s0y[kTile], s0z[kTile];
-    __shared__ double sq[kTile], sa[kTile], sze[kTile], ssz[kTile];
+    __shared__ double sq[kTile], sa[kTile], ssz[kTile];
     __shared__ double sw0[7][kTile], sw[7][kTile];
-    __shared__ int ssl[kTile], snr[kTile];
+    __shared__ int sko[kTile], snr[kTile];
     const int i0 = blockIdx.x * kTile, i = i0 + threadIdx.x;
     int jb, je;
     tile_range(V, i0, nsplit, jb, je);
     const bool act = i < V.n;
     const int ic = act ? i : i0;
     const double4 pi = V.pos[ic], p0i = V.pos0[ic];
-    const double ai = V.alpeeq[ic], qi = V.q[ic], zi = V.zeta[ic], szi = V.szr[ic];
+    const double ai = V.alpeeq[ic], qi = V.q[ic], szi = V.szr[ic];
     const int2 rg = act ? V.jr[i] : make_int2(0, 0);
-    const double* g0i = V.g0 + (size_t)ic * V.K * 7;
-    const double* dgi = V.hdg + (size_t)ic * V.K * 7;
+    const int rowi = ic + V.pshift[V.mol[ic]];
     const double tsp = 2.0 / 1.772453850905516;
     double ec = 0.0, ed = 0.0, gx = 0.0, gy = 0.0, gz = 0.0, dcn = 0.0, cfar = 0.0;
     for (int t0 = jb; t0 < je; t0 += kTile) {
@@ -350,12 +359,12 @@ __global__ void __launch_bounds__(kTile) k_pairs(View V, int nsplit)
             const double4 p = V.pos[jl], p0 = V.pos0[jl];
             sx[u] = p.x; sy[u] = p.y; sz[u] = p.z;
             s0x[u] = p0.x; s0y[u] = p0.y; s0z[u] = p0.z;
-            sq[u] = V.q[jl]; sa[u] = V.alpeeq[jl]; sze[u] = V.zeta[jl]; ssz[u] = V.szr[jl];
-            ssl[u] = V.slot[jl]; snr[u] = V.nref[jl];
-#pragma unroll
-            for (int b = 0; b < 7; ++b) {
-                sw0[b][u] = V.w0[(size_t)jl * 7 + b];
-                sw[b][u] = V.w[(size_t)jl * 7 + b];
+            sq[u] = V.q[jl]; sa[u] = V.alpeeq[jl]; ssz[u] = V.szr[jl];
+            sko[u] = V.kof[jl]; snr[u] = V.nref[jl];
+            const int row = jl + V.pshift[V.mol[jl]];
+            for (int b = 0; b < snr[u]; ++b) {
+                sw0[b][u] = V.w0p[pk(V.Rp, row, sko[u] + b)];
+                sw[b][u] = V.wp[pk(V.Rp, row, sko[u] + b)];
             }
         }
         __syncthreads();
@@ -390,15 +399,8 @@ __global__ void __launch_bounds__(kTile) k_pairs(View V, int nsplit)
             }
             if (d2 <= 2500.0 &&
                 d2_exact(p0i, make_double4(s0x[jj], s0y[jj], s0z[jj], 0.0)) <= 3600.0) {
-                const int sj = ssl[jj], nr = snr[jj];
-                const double* g0 = g0i + sj * 7;
-                const double* dg = dgi + sj * 7;
                 double e, dedr, dc;
-                // mixed form: pairs closer than 15 bohr (the strong ones) stay FP64
-                if (sizeof(R) == sizeof(double) || d2 < 225.0)
-                    d4_pair<double>(d2, g0, dg, sw0, sw, jj, nr, szi, ssz[jj], zi * sze[jj], e, dedr, dc);
-                else
-                    d4_pair<R>(d2, g0, dg, sw0, sw, jj, nr, szi, ssz[jj], zi * sze[jj], e, dedr, dc);
+                d4_pair(V, d2, rowi, sko[jj], sw0, sw, jj, snr[jj], szi, ssz[jj], e, dedr, dc);
                 ed += e;
                 f += dedr;
                 if (!V.exact) dcn += dc;
@@ -416,244 +418,6 @@ __global__ void __launch_bounds__(kTile) k_pairs(View V, int nsplit)
     const int m = act ? V.mol[i] : -1;
     eadd(V, 0.5 * ec, m, T_COUL);
     eadd(V, 0.5 * ed, m, T_DISP);
-}
-
-// ------------------------------------------------------------------------------------
-// The same Coulomb + D4 pair terms with every pair evaluated once (Newton's third law).
-// Blocks take T x T tiles (i tile <= j tile, listed at set-up; only j > i within a
-// diagonal tile; T = 64 for single molecules, 32 for batches of small molecules, whose
-// tiles would otherwise straddle molecules).  Row i keeps its sums in registers as in k_pairs; the j side of every
-// pair (gradient, dE/dCN_j from j's half contraction against i's current weights, and the
-// far-pair potential of the exact-gradient mode) is summed over the warp's 32 rows with
-// shuffles and kept per warp in shared memory, then added once per tile.
-// ------------------------------------------------------------------------------------
-constexpr int kST = 64;
-
-// one D4 pair in arithmetic type R with both CN derivatives: energy e, dE/dr / r in dedr,
-// dE/dCN_i in dci, dE/dCN_j in dcj (wi: current weights of i in registers)
-template <class R, int T>
-__device__ __forceinline__ void d4_pair_sym(double d2, const double* g0, const double* dgi, const double* dgj,
-                                            const double (*sw0)[T], const double (*sw)[T], int jj, int nrj,
-                                            int nri, const double (&wi)[7], double r4r2_d, double sr4r2_d,
-                                            double zz_d, bool want_dc, double& e, double& dedr, double& dci,
-                                            double& dcj)
-{
-    R c6 = R(0), dc6i = R(0), dc6j = R(0);
-    for (int b = 0; b < nrj; ++b) c6 += (R)__ldg(g0 + b) * (R)sw0[b][jj];
-    if (want_dc) {
-        for (int b = 0; b < nrj; ++b) dc6i += (R)__ldg(dgi + b) * (R)sw[b][jj];
-#pragma unroll
-        for (int a = 0; a < 7; ++a)
-            if (a < nri) dc6j += (R)__ldg(dgj + a) * (R)wi[a];
-    }
-    const R q2 = (R)d2;
-    const R r4r2 = (R)r4r2_d;
-    const R t = R(0.58) * (R)sr4r2_d + R(4.80);   // sr4r2_d = sqrt(r4r2) from per-atom roots
-    const R r0sq = t * t;
-    const R zz = (R)zz_d;
-    const R r6 = q2 * q2 * q2, r06 = r0sq * r0sq * r0sq;
-    // 1/a and 1/b from one division: a*b stays below 1e24 for r <= 50 bohr
-    const R a6 = r6 + r06, a8 = r6 * q2 + r06 * r0sq;
-    const R inv = R(1) / (a6 * a8);
-    const R t6 = a8 * inv, t8 = a6 * inv;
-    const R sum = t6 + R(2) * r4r2 * t8;
-    e = -(double)(c6 * sum * zz);
-    const R d6 = R(-6) * q2 * q2 * t6 * t6, d8 = R(-8) * r6 * t8 * t8;
-    dedr = -(double)(c6 * zz * (d6 + R(2) * r4r2 * d8));
-    dci = -(double)(dc6i * sum * zz);
-    dcj = -(double)(dc6j * sum * zz);
-}
-
-// PART selects the terms: kPairCoul (needs this step's charges), kPairD4 (needs only the
-// CN weights, so it can run beside the EEQ solve), or both in one pass
-constexpr int kPairCoul = 1, kPairD4 = 2, kPairBoth = 3;
-template <class R, int MINB, int T, int PART>
-__global__ void __launch_bounds__(T, MINB) k_pairs_sym(View V, const int2* __restrict__ tiles)
-{
-    constexpr bool COUL = (PART & kPairCoul) != 0, D4 = (PART & kPairD4) != 0;
-    constexpr int NA = 5;   // j-side sums: fx, fy, fz, dE/dCN_j (D4), far potential (Coulomb)
-    __shared__ double sx[T], sy[T], sz[T];
-    __shared__ double sq[COUL ? T : 1], sa[COUL ? T : 1];
-    __shared__ double s0x[D4 ? T : 1], s0y[D4 ? T : 1], s0z[D4 ? T : 1];
-    __shared__ double sze[D4 ? T : 1], ssz[D4 ? T : 1], srz[D4 ? T : 1];
-    __shared__ double sw0[D4 ? 7 : 1][T], sw[D4 ? 7 : 1][T];
-    __shared__ int ssl[D4 ? T : 1], snr[D4 ? T : 1];
-    __shared__ double jacc[T / 32][NA][T];
-    const int2 tp = tiles[blockIdx.x];
-    const int i0 = tp.x, j0 = tp.y, i = i0 + threadIdx.x;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const bool act = i < V.n;
-    const int ic = act ? i : i0;
-    const double4 pi = V.pos[ic];
-    const int2 rg = act ? V.jr[i] : make_int2(0, 0);
-    double ai = 0.0, qi = 0.0;
-    if constexpr (COUL) { ai = V.alpeeq[ic]; qi = V.q[ic]; }
-    double4 p0i = make_double4(0.0, 0.0, 0.0, 0.0);
-    double zi = 0.0, szi = 0.0, s3i = 0.0;
-    int si = 0, nri = 0;
-    double wi[7];
-    const double* g0i = nullptr;
-    const double* dgi = nullptr;
-    if constexpr (D4) {
-        p0i = V.pos0[ic];
-        zi = V.zeta[ic]; szi = V.szr[ic];
-        s3i = sqrt(3.0 * szi);   // sqrt(r4r2) of a pair = s3i * sqrt(szr_j)
-        si = V.slot[ic]; nri = V.nref[ic];
-#pragma unroll
-        for (int a = 0; a < 7; ++a) wi[a] = V.w[(size_t)ic * 7 + a];
-        g0i = V.g0 + (size_t)ic * V.K * 7;
-        dgi = V.hdg + (size_t)ic * V.K * 7;
-    }
-    const bool want_dc = !V.exact, want_far = COUL && V.cfar != nullptr;
-    {
-        const int jl = j0 + threadIdx.x;
-        if (jl < V.n) {
-            const int u = threadIdx.x;
-            const double4 p = V.pos[jl];
-            sx[u] = p.x; sy[u] = p.y; sz[u] = p.z;
-            if constexpr (COUL) { sq[u] = V.q[jl]; sa[u] = V.alpeeq[jl]; }
-            if constexpr (D4) {
-                const double4 p0 = V.pos0[jl];
-                s0x[u] = p0.x; s0y[u] = p0.y; s0z[u] = p0.z;
-                sze[u] = V.zeta[jl]; ssz[u] = V.szr[jl]; srz[u] = sqrt(ssz[u]);
-                ssl[u] = V.slot[jl]; snr[u] = V.nref[jl];
-#pragma unroll
-                for (int b = 0; b < 7; ++b) {
-                    sw0[b][u] = V.w0[(size_t)jl * 7 + b];
-                    sw[b][u] = V.w[(size_t)jl * 7 + b];
-                }
-            }
-        }
-    }
-    // j-side sums, per warp in shared memory, in two passes over the tile's partners.
-    // Coulomb pass: at step k lane t of the block takes partner (t + k) mod T, so the lanes of
-    // a warp always hold distinct partners and add their j-side terms without shuffles or
-    // conflicts (1000 waters, Coulomb launch: 104 -> 53 us against warp-wide reductions).
-    // D4 pass: the lanes take the same partner and the j-side sums are reduced over the warp
-    // (rotated partners made the per-partner reference loops diverge: D4 61 -> 122 us); a
-    // warp runs it only when one of its pairs is within the 50 bohr D4 range, which the
-    // Coulomb pass records.
-#pragma unroll
-    for (int k = 0; k < NA; ++k)
-        for (int u = lane; u < T; u += 32) jacc[warp][k][u] = 0.0;
-    __syncthreads();
-    const double tsp = 2.0 / 1.772453850905516;
-    double ec = 0.0, ed = 0.0, gx = 0.0, gy = 0.0, gz = 0.0, dcn = 0.0, cfar = 0.0;
-    const int cnt = min(T, V.n - j0);
-    bool near = !COUL;   // a pair within the D4 range (D4-only launches: assume one)
-    if constexpr (COUL) {
-        for (int k = 0; k < T; ++k) {
-            const int jj = (threadIdx.x + k) & (T - 1);
-            if (jj >= cnt) continue;
-            const int j = j0 + jj;
-            if (!(act && j > i && j >= rg.x && j < rg.y)) continue;
-            double dx = pi.x - sx[jj], dy = pi.y - sy[jj], dz = pi.z - sz[jj];
-            if (V.cell.on) mic(V.cell, dx, dy, dz);
-            const double d2 = dx * dx + dy * dy + dz * dz;
-            if (!(d2 >= 1e-20)) continue;
-            double f = 0.0, cfj = 0.0;   // dE/dr / r
-            if (d2 <= 10000.0) {
-                const double s = ai + sa[jj];
-                const double qq = qi * sq[jj];
-                if (d2 >= 36.0 * s) {
-                    const double ir = rsqrt(d2);
-                    const double e = qq * ir;
-                    ec += e;
-                    f -= e * ir * ir;
-                } else {
-                    const double r = sqrt(d2);
-                    const double g = 1.0 / sqrt(s);
-                    const double gr = g * r;
-                    const double ef = erf(gr);
-                    ec += qq * ef / r;
-                    f += qq * ((g * exp(-gr * gr) * tsp) / r - ef / d2) / r;
-                }
-            } else if (want_far) {
-                const double ir = rsqrt(d2);   // cut pair: its EEQ element is 1/r
-                cfar += sq[jj] * ir;
-                cfj = qi * ir;
-            }
-            if (D4) near |= d2 <= 2500.0;
-            gx += f * dx; gy += f * dy; gz += f * dz;
-            jacc[warp][0][jj] -= f * dx;
-            jacc[warp][1][jj] -= f * dy;
-            jacc[warp][2][jj] -= f * dz;
-            if (want_far) jacc[warp][4][jj] += cfj;
-        }
-    }
-    if constexpr (D4) {
-        if (__any_sync(0xffffffffu, near)) {
-            for (int k = 0; k < cnt; ++k) {
-                const int jj = k;
-                const int j = j0 + jj;
-                double fx = 0.0, fy = 0.0, fz = 0.0, dcj = 0.0;
-                bool hit = false;   // this lane has a j-side contribution
-                if (act && j > i && j >= rg.x && j < rg.y) {
-                    double dx = pi.x - sx[jj], dy = pi.y - sy[jj], dz = pi.z - sz[jj];
-                    if (V.cell.on) mic(V.cell, dx, dy, dz);
-                    const double d2 = dx * dx + dy * dy + dz * dz;
-                    if (d2 >= 1e-20 && d2 <= 2500.0 &&
-                        d2_exact(p0i, make_double4(s0x[jj], s0y[jj], s0z[jj], 0.0)) <= 3600.0) {
-                        hit = true;
-                        const int sj = ssl[jj], nrj = snr[jj];
-                        const double* dgj = V.hdg + ((size_t)j * V.K + si) * 7;
-                        const double r4r2 = 3.0 * szi * ssz[jj], sr4r2 = s3i * srz[jj], zz = zi * sze[jj];
-                        double e, dedr, dci;
-                        // mixed form: pairs closer than 15 bohr (the strong ones) stay FP64
-                        if (sizeof(R) == sizeof(double) || d2 < 225.0)
-                            d4_pair_sym<double, T>(d2, g0i + sj * 7, dgi + sj * 7, dgj, sw0, sw, jj, nrj, nri, wi,
-                                                   r4r2, sr4r2, zz, want_dc, e, dedr, dci, dcj);
-                        else
-                            d4_pair_sym<R, T>(d2, g0i + sj * 7, dgi + sj * 7, dgj, sw0, sw, jj, nrj, nri, wi, r4r2,
-                                              sr4r2, zz, want_dc, e, dedr, dci, dcj);
-                        ed += e;
-                        dcn += dci;
-                        gx += dedr * dx; gy += dedr * dy; gz += dedr * dz;
-                        fx = -dedr * dx; fy = -dedr * dy; fz = -dedr * dz;
-                    }
-                }
-                if (__any_sync(0xffffffffu, hit)) {
-                    for (int o = 16; o > 0; o >>= 1) {
-                        fx += __shfl_xor_sync(0xffffffffu, fx, o);
-                        fy += __shfl_xor_sync(0xffffffffu, fy, o);
-                        fz += __shfl_xor_sync(0xffffffffu, fz, o);
-                    }
-                    if (want_dc)
-                        for (int o = 16; o > 0; o >>= 1) dcj += __shfl_xor_sync(0xffffffffu, dcj, o);
-                    if (lane == 0) {
-                        jacc[warp][0][jj] += fx; jacc[warp][1][jj] += fy; jacc[warp][2][jj] += fz;
-                        jacc[warp][3][jj] += dcj;
-                    }
-                }
-            }
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < cnt) {
-        const int j = j0 + threadIdx.x;
-        double a[NA];
-#pragma unroll
-        for (int k = 0; k < NA; ++k) {
-            a[k] = 0.0;
-#pragma unroll
-            for (int w = 0; w < T / 32; ++w) a[k] += jacc[w][k][threadIdx.x];
-        }
-        if (a[0] != 0.0) atomicAdd(V.grad + 3 * j, a[0]);
-        if (a[1] != 0.0) atomicAdd(V.grad + 3 * j + 1, a[1]);
-        if (a[2] != 0.0) atomicAdd(V.grad + 3 * j + 2, a[2]);
-        if (a[3] != 0.0) atomicAdd(V.dEdcn + j, a[3]);
-        if (a[4] != 0.0) atomicAdd(V.cfar + j, a[4]);
-    }
-    if (act) {
-        if (gx != 0.0) atomicAdd(V.grad + 3 * i, gx);
-        if (gy != 0.0) atomicAdd(V.grad + 3 * i + 1, gy);
-        if (gz != 0.0) atomicAdd(V.grad + 3 * i + 2, gz);
-        if (dcn != 0.0) atomicAdd(V.dEdcn + i, dcn);
-        if (cfar != 0.0) atomicAdd(V.cfar + i, cfar);
-    }
-    const int m = act ? V.mol[i] : -1;
-    if constexpr (COUL) eadd(V, ec, m, T_COUL);
-    if constexpr (D4) eadd(V, ed, m, T_DISP);
 }
 
 // ------------------------------------------------------------------------------------

@@ -649,39 +649,12 @@ __device__ double matvec_tiles64(const PCGArgs& A, const double* p, double* red)
 constexpr int kPcgHalf = 64 * kPcgT;   // floats of half a tile
 constexpr int kPcgStages = 4;          // halves in flight
 constexpr int kPcgStageF = kPcgHalf + kPcgT + 64;   // floats per stage: elements, pr, pc
-constexpr long long kTmaPolls = 1ll << 24;
 
 __host__ __device__ inline int pcg_ir_pregion(int n)
 {
     const int pd = (n + 1) & ~1;
     const int ring = kPcgStages * kPcgStageF / 2 + 16;   // doubles, with room to align to 128 bytes
     return pd > ring ? pd : ring;
-}
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-// true once the phase with the given parity has completed; false after kTmaPolls polls
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity)
-{
-    for (long long k = 0; k < kTmaPolls; ++k) {
-        unsigned done;
-        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                     " selp.u32 %0, 1, 0, p;\n}\n"
-                     : "=r"(done)
-                     : "r"(smem_u32(bar)), "r"(parity)
-                     : "memory");
-        if (done) return true;
-    }
-    return false;
 }
 
 // TMA of half h's elements (box 128 rows x 64 columns at rows I0, columns J0 + 64 half) and

@@ -1,0 +1,68 @@
+"""The tiled Coulomb and D4 pair kernels at the edges of their tiles (32 rows, 8 partners a step,
+16 to 64 partners a tile), against the oracle: sizes around the multiples, every tile shape, and
+a geometry far from the set-up, where the D4 list membership is tested pair by pair.
+
+Tolerances: both sides sum FP64 terms of at most ~1 Eh over n^2 / 2 < 1e4 pairs (rounding below
+1e-12); the charges are solved to a residual of 1e-12 of the right-hand side, which moves the
+energies by its square and the gradient by about 1e-12."""
+import numpy as np
+import pytest
+
+from curcuma_b200 import FP64, GFNFF, workloads
+from tests.oracle_api import Oracle
+
+pytestmark = pytest.mark.gpu
+
+VARIANTS = ["sym32", "sym64", "sym64_occ10"]
+
+
+def _compare(Z, X, variant, monkeypatch):
+    monkeypatch.setenv("GFNFF_PAIRS_VARIANT", variant)
+    g = GFNFF(precision=FP64)
+    assert g.setMolecule(Z, X), g.getErrorMessage()
+    e = g.calculateEnergy(True)
+    assert not g.hasError(), g.getErrorMessage()
+    T, G, q, cn = Oracle(Z, X).engrad(X)
+    D = g.getEnergyDecomposition()
+    assert abs(D["coulomb"] - T["coulomb"]) < 1e-10
+    assert abs(D["dispersion"] - T["dispersion"]) < 1e-10
+    assert abs(e - T["total"]) < 1e-10
+    assert np.abs(g.getGradient() - G).max() < 1e-10
+    return g, e
+
+
+@pytest.mark.parametrize("variant", VARIANTS)
+@pytest.mark.parametrize("n_water", [1, 5, 10, 11, 21, 22, 43])   # 3 .. 129 atoms: 30|33, 63|66, 129
+def test_tile_edges_water(n_water, variant, monkeypatch):
+    _compare(*workloads.water_cluster(n_water, 100 + n_water), variant, monkeypatch)
+
+
+@pytest.mark.parametrize("variant", VARIANTS)
+@pytest.mark.parametrize("size", [24, 31, 40, 65, 97])   # C/H/N/O: 17 packed references
+def test_tile_edges_chain(size, variant, monkeypatch):
+    _compare(*workloads.random_chain(size, np.random.default_rng(size)), variant, monkeypatch)
+
+
+def test_far_from_setup(monkeypatch):
+    Z, X = workloads.water_cluster(20, 3)
+    g, e = _compare(Z, X, "sym32", monkeypatch)
+    g0 = g.getGradient()
+    g.updateGeometry(X + np.array([4.0, -2.0, 1.0]))   # 7.6 bohr: beyond the free displacement
+    assert abs(g.calculateEnergy(True) - e) < 1e-9
+    assert np.abs(g.getGradient() - g0).max() < 1e-9
+
+
+def test_batch_of_ragged_molecules(monkeypatch):
+    rng = np.random.default_rng(8)
+    mols = [workloads.random_chain(n, rng) for n in (20, 33, 64, 70)] + [workloads.water_cluster(1, 2)]
+    for variant in VARIANTS:
+        monkeypatch.setenv("GFNFF_PAIRS_VARIANT", variant)
+        g = GFNFF(precision=FP64)
+        assert g.setMoleculeBatch(mols), g.getErrorMessage()
+        e, st = g.calculateEnergyBatch()
+        assert (st == 0).all()
+        G = np.split(g.getGradient(), np.cumsum([len(z) for z, _ in mols])[:-1])
+        for (Z, X), em, gm in zip(mols, e, G):
+            T, Go, q, cn = Oracle(Z, X).engrad(X)
+            assert abs(em - T["total"]) < 1e-10
+            assert np.abs(gm - Go).max() < 1e-10
