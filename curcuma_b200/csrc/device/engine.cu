@@ -55,6 +55,7 @@ namespace gfnff {
 #include "k_alpb.cuh"
 #include "k_eeq.cuh"
 #include "k_eeq_tc.cuh"
+#include "k_eeq_cg.cuh"
 #include "k_chol.cuh"
 #include "k_pcg.cuh"
 #include "k_lu.cuh"
@@ -432,6 +433,161 @@ struct Engine::Impl {
     DBuf<int> refine;      // largest number of refinement corrections of the last launch
     DBuf<int4> tc_tiles;   // {molecule, R, C} of every FP64 tile (k_eeq_tc_tiles)
     int n_tc_tiles = 0;
+    // batched EEQ by conjugate gradients (k_eeq_cg): set-up inverses, and the molecules of every
+    // launch (bin): cluster size, dynamic shared memory.  The bins run on streams of their own.
+    bool cg_on = false;
+    DBuf<float> cg_pinv;
+    DBuf<long long> cg_poff;
+    struct CgBin {
+        int cs = 1, first = 0, count = 0, threads = 64;
+        size_t smem = 0, inv_smem = 0;
+    };
+    std::vector<CgBin> cg_bins;
+    DBuf<int> cg_mols, cg_iters;
+    std::vector<cudaStream_t> cg_streams;
+    std::vector<cudaEvent_t> cg_done;
+    cudaEvent_t cg_fork = nullptr;
+    // bins of the molecules with nr unknowns and na atoms each
+    void plan_cg(const std::vector<int>& nr, const std::vector<int>& na)
+    {
+        cg_bins.clear();
+        const size_t cap = 208 * 1024;
+        // a factorisation's time is that of its longest molecule until the chip is full, CG's grows
+        // with the number of CTAs from the start: 200 conformers (2.0 waves of CTAs) take 165 / 195
+        // us (mixed / FP64) against 255 / 510, 512 (5.1 waves) 393 / 453 against 306 / 666
+        const double waves = opt.precision == 1 ? 3.0 : 8.0;
+        const int nm = (int)nr.size();
+        std::vector<int> cs(nm, 1);
+        int ctas = 0;
+        double slots = 0.0;   // SMs' worth of CTAs
+        for (int m = 0; m < nm; ++m) {
+            while (cs[m] < 8 && cg_smem(nr[m], na[m], cs[m]) > cap) cs[m] *= 2;
+            if (cg_smem(nr[m], na[m], cs[m]) > cap) return;   // cg_on stays false
+            ctas += cs[m];
+            slots += cs[m] > 1 ? cs[m] : std::max(1.0 / 8.0, cg_smem(nr[m], na[m], 1) / 222e3);
+        }
+        if (slots > waves * 148.0) return;
+        // few molecules: larger clusters while the SMs hold one CTA each (a product and the
+        // build shrink with the slice; below ~48 unknowns the barriers cost more)
+        for (int top = 2; top <= 4; top *= 2) {
+            int more = 0;
+            for (int m = 0; m < nm; ++m) more += nr[m] > 24 * top && cs[m] < top ? top - cs[m] : 0;
+            if (ctas + more > 148) break;
+            for (int m = 0; m < nm; ++m)
+                if (nr[m] > 24 * top && cs[m] < top) cs[m] = top;
+            ctas += more;
+        }
+        // one bin per cluster size, single CTAs also by the number that fits an SM
+        auto bin_of = [&](int m) {
+            const size_t b = cg_smem(nr[m], na[m], cs[m]);
+            return cs[m] > 1 ? cs[m] * 16 : (b <= 24 * 1024 ? 0 : (b <= 54 * 1024 ? 1 : (b <= 110 * 1024 ? 2 : 3)));
+        };
+        std::map<int, std::vector<int>> by;
+        for (int m = 0; m < nm; ++m) by[bin_of(m)].push_back(m);
+        std::vector<int> mols;
+        for (auto it = by.rbegin(); it != by.rend(); ++it) {   // the largest clusters first
+            CgBin b;
+            b.cs = cs[it->second[0]];
+            b.first = (int)mols.size();
+            std::stable_sort(it->second.begin(), it->second.end(), [&](int x, int y) { return nr[x] > nr[y]; });
+            for (int m : it->second) {
+                mols.push_back(m);
+                b.smem = std::max(b.smem, cg_smem(nr[m], na[m], b.cs));
+                b.inv_smem = std::max(b.inv_smem, gfnff::inv_smem(nr[m], na[m], b.cs));
+                b.threads = std::max(b.threads, cg_threads(nr[m], b.cs));
+            }
+            b.count = (int)mols.size() - b.first;
+            cg_bins.push_back(b);
+        }
+        cg_mols.upload(mols);
+        cg_iters.alloc(1);
+        std::vector<long long> off(nm);
+        long long tot = 0;
+        for (int m = 0; m < nm; ++m) {
+            off[m] = tot;
+            tot += (long long)nr[m] * cg_ld(nr[m]);
+        }
+        cg_poff.upload(off);
+        cg_pinv.alloc((size_t)std::max<long long>(1, tot));
+        allow_smem((const void*)k_eeq_cg<1>, cap);
+        allow_smem((const void*)k_eeq_cg<2>, cap);
+        allow_smem((const void*)k_eeq_cg<4>, cap);
+        allow_smem((const void*)k_eeq_cg<8>, cap);
+        allow_smem((const void*)k_eeq_inv<1>, cap);
+        allow_smem((const void*)k_eeq_inv<2>, cap);
+        allow_smem((const void*)k_eeq_inv<4>, cap);
+        allow_smem((const void*)k_eeq_inv<8>, cap);
+        int lo = 0, hi = 0;
+        CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+        while (cg_streams.size() + 1 < cg_bins.size()) {
+            cudaStream_t st;
+            cudaEvent_t e;
+            CK(cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, hi));
+            cg_streams.push_back(st);
+            CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+            cg_done.push_back(e);
+        }
+        if (!cg_fork) CK(cudaEventCreateWithFlags(&cg_fork, cudaEventDisableTiming));
+        cg_on = true;
+    }
+    CgArgs cg_args() const
+    {
+        // a batch leaves unsolved molecules to k_eeq_batch (-1), a single molecule to the host
+        return CgArgs{cg_mols.p, roff.p, red2atom.p, anchor.p, qlist.p, nq, q0.p, cg_pinv.p, cg_poff.p, bvec.p, info.p,
+                      nmol > 1 ? -1 : 1, nmol > 1 ? -1 : 3, cg_iters.p, 500, opt.precision == 1 ? kRefineTol : 0.0};
+    }
+    // one cluster of b.cs CTAs per molecule of the bin
+    template <class... P, class... Q>
+    void cg_go(void (*kernel)(P...), const CgBin& b, int threads, size_t smem, cudaStream_t st, Q... args)
+    {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(b.count * b.cs);
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = b.cs;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        CK(cudaLaunchKernelEx(&cfg, kernel, args...));
+    }
+    // inverses of the reduced matrices at the geometry in pos
+    void cg_invert()
+    {
+        if (!cg_on) return;
+        CgArgs A = cg_args();
+        for (const CgBin& b : cg_bins) {
+            A.mols = cg_mols.p + b.first;
+            switch (b.cs) {
+            case 1: cg_go(k_eeq_inv<1>, b, 512, b.inv_smem, stream, view(), A, cg_pinv.p); break;
+            case 2: cg_go(k_eeq_inv<2>, b, 512, b.inv_smem, stream, view(), A, cg_pinv.p); break;
+            case 4: cg_go(k_eeq_inv<4>, b, 512, b.inv_smem, stream, view(), A, cg_pinv.p); break;
+            default: cg_go(k_eeq_inv<8>, b, 512, b.inv_smem, stream, view(), A, cg_pinv.p);
+            }
+        }
+    }
+    void cg_launch(const View& V, cudaStream_t s)
+    {
+        CK(cudaMemsetAsync(cg_iters.p, 0, sizeof(int), s));
+        CgArgs A = cg_args();
+        if (cg_bins.size() > 1) CK(cudaEventRecord(cg_fork, s));
+        for (size_t k = 0; k < cg_bins.size(); ++k) {
+            const CgBin& b = cg_bins[k];
+            cudaStream_t st = k == 0 ? s : cg_streams[k - 1];
+            if (k) CK(cudaStreamWaitEvent(st, cg_fork, 0));
+            A.mols = cg_mols.p + b.first;
+            switch (b.cs) {
+            case 1: cg_go(k_eeq_cg<1>, b, b.threads, b.smem, st, V, A); break;
+            case 2: cg_go(k_eeq_cg<2>, b, b.threads, b.smem, st, V, A); break;
+            case 4: cg_go(k_eeq_cg<4>, b, b.threads, b.smem, st, V, A); break;
+            default: cg_go(k_eeq_cg<8>, b, b.threads, b.smem, st, V, A);
+            }
+            if (k) CK(cudaEventRecord(cg_done[k - 1], st));
+        }
+        for (size_t k = 1; k < cg_bins.size(); ++k) CK(cudaStreamWaitEvent(s, cg_done[k - 1], 0));
+    }
     // bonded lists
     DBuf<int> b_i, b_j, b_h, b_off, b_hb;
     DBuf<double> b_fc, b_al, b_r0i, b_r0j, b_cki, b_ckj, b_sh, b_ff;
@@ -813,6 +969,9 @@ Engine::~Engine()
     if (p_->cnl_bad_host) cudaFreeHost(p_->cnl_bad_host);
     for (cudaEvent_t e : {p_->ev_fork0, p_->ev_fork1, p_->ev_join, p_->ev_join_d4})
         if (e) cudaEventDestroy(e);
+    for (cudaStream_t st : p_->cg_streams) cudaStreamDestroy(st);
+    for (cudaEvent_t e : p_->cg_done) cudaEventDestroy(e);
+    if (p_->cg_fork) cudaEventDestroy(p_->cg_fork);
     if (p_->side) cudaStreamDestroy(p_->side);
     if (p_->side_d4) cudaStreamDestroy(p_->side_d4);
     if (p_->stream) cudaStreamDestroy(p_->stream);
@@ -1261,6 +1420,17 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
         // batches, and single molecules small enough for the batched kernel's staging
         // (a candidate EEQ solver for them)
         P.batch_ready = nm > 1 || n <= kStageAtoms;
+        P.cg_on = false;
+        // GFNFF_BATCH_TC=0: the FP64 Cholesky for every molecule
+        const char* ecg = std::getenv("GFNFF_BATCH_TC");
+        if (P.batch_ready && P.nred > 0 && !(ecg && !std::strcmp(ecg, "0"))) {
+            std::vector<int> nr(nm), na(nm);
+            for (int m = 0; m < nm; ++m) {
+                nr[m] = roff[m + 1] - roff[m];
+                na[m] = mols[m]->n;
+            }
+            P.plan_cg(nr, na);
+        }
         if (P.batch_ready) {
             std::vector<int> ord(nm);
             std::iota(ord.begin(), ord.end(), 0);
@@ -1271,7 +1441,7 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
             // mixed form: the tensor-core path (k_eeq_tc.cuh) for every molecule of at most
             // kTcMaxRed unknowns (GFNFF_BATCH_TC=0: the FP64 paths)
             const char* etc = std::getenv("GFNFF_BATCH_TC");
-            P.batch_tc = P.opt.precision == 1 && !(etc && !std::strcmp(etc, "0"));
+            P.batch_tc = P.opt.precision == 1 && !P.cg_on && !(etc && !std::strcmp(etc, "0"));
             // work items: large molecules one per block, small ones in packs of kWarpMols
             // (one warp each, FP64); in the mixed form every molecule is a block item (one
             // small molecule on a block's tensor-core path measured far below a warp item of
@@ -1805,6 +1975,15 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
     const bool graphs_setting = P.graphs_ok;
     P.graphs_ok = false;   // probes below run direct (their buffers are temporary)
     P.pcg_warm = false;    // and PCG probes start from zero
+    if (nm > 1 && P.cg_on) {
+        std::vector<double> h;
+        for (const Model* m : mols) h.insert(h.end(), m->xyz_setup.begin(), m->xyz_setup.end());
+        DBuf<double> x;
+        x.upload(h);
+        launch_positions(x.p, true);
+        P.cg_invert();
+        CK(cudaStreamSynchronize(P.stream));
+    }
     if (nm == 1 && P.nred > 0) {
         DBuf<double> x;
         std::vector<double> h(mols[0]->xyz_setup);
@@ -1815,6 +1994,7 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
         int st = 0;
         fetch(nullptr, nullptr, &st, nullptr);
         if (st == GFNFF_NOT_SPD) P.use_lu = true;
+        else P.cg_invert();   // positions and Born radii are those of the set-up geometry
         // Solver: GFNFF_EEQ_SOLVER=library|tiled|pcg|batched forces one; otherwise the fastest
         // of the in-house ones (tiled, pcg, batched) over three evaluations at the setup
         // geometry.  cuSOLVER ("library") is an explicit opt-in only.
@@ -1824,14 +2004,14 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
             if (env && !std::strcmp(env, "library")) cand = {Impl::SOLVE_LIBRARY};
             else if (env && !std::strcmp(env, "tiled")) cand = {Impl::SOLVE_TILED};
             else if (env && !std::strcmp(env, "pcg") && P.pcg_ready) cand = {Impl::SOLVE_PCG};
-            else if (env && !std::strcmp(env, "batched") && P.batch_ready && !P.resp_on && !P.alpb_on)
+            else if (env && !std::strcmp(env, "batched") && P.batch_ready && !P.resp_on && (!P.alpb_on || P.cg_on))
                 cand = {Impl::SOLVE_BATCH};
             else {
                 cand = {Impl::SOLVE_TILED};
                 if (P.pcg_ready) cand.push_back(Impl::SOLVE_PCG);
-                // the batched kernel keeps no factor for the charge-response solve
-                // (nor the solvent's Born matrix: it builds its matrix from the atoms)
-                if (P.batch_ready && !P.resp_on && !P.alpb_on) cand.push_back(Impl::SOLVE_BATCH);
+                // the batched kernels keep no factor for the charge-response solve; the Cholesky one
+                // builds its matrix without the solvent's Born term
+                if (P.batch_ready && !P.resp_on && (!P.alpb_on || P.cg_on)) cand.push_back(Impl::SOLVE_BATCH);
             }
             if (cand.size() == 1) {
                 P.solver = cand[0];
@@ -1977,7 +2157,7 @@ bool Engine::switch_to_lu()
 bool Engine::switch_to_direct()
 {
     if (p_->nmol != 1) return false;
-    if (p_->solver != Impl::SOLVE_PCG && !(p_->solver == Impl::SOLVE_BATCH && p_->batch_tc)) return false;
+    if (p_->solver != Impl::SOLVE_PCG && !(p_->solver == Impl::SOLVE_BATCH && (p_->batch_tc || p_->cg_on))) return false;
     p_->drop_graphs();
     p_->solver = Impl::SOLVE_TILED;   // the in-house FP64 Cholesky
     return true;
@@ -2007,6 +2187,12 @@ int Engine::eeq_fp64_products()
 int Engine::eeq_iterations()
 {
     const bool batched = p_->nmol != 1 || (!p_->use_lu && p_->solver == Impl::SOLVE_BATCH);
+    if (batched && p_->cg_on) {   // products of the slowest molecule
+        int it = 0;
+        CK(cudaStreamSynchronize(p_->stream));
+        CK(cudaMemcpy(&it, p_->cg_iters.p, sizeof(int), cudaMemcpyDeviceToHost));
+        return it;
+    }
     if (batched && p_->batch_tc) {   // refinement corrections of the tensor-core path
         int it = 0;
         CK(cudaStreamSynchronize(p_->stream));
@@ -2268,14 +2454,17 @@ void Engine::launch_body()
         P.mark(5);
         CK(cudaMemsetAsync(P.bnext.p, 0, sizeof(int), s));
         if (fork && !early) CK(cudaEventRecord(P.ev_fork1, s));   // single molecule, batched solver
-        EEQBatch B{P.roff.p, P.moff.p, P.border.p, P.bitems.p, P.nbitems, P.bnext.p, P.batch_smem_max, P.red2atom.p,
-                   P.anchor.p, P.qlist.p, P.nq, P.q0.p, P.M.p, P.bvec.p, P.info.p,
-                   P.batch_tc ? 1 : 0, P.M64.p, P.m64off.p, kRefineTol, P.refine.p};
-        if (P.batch_tc) {
-            CK(cudaMemsetAsync(P.refine.p, 0, sizeof(int), s));
-            if (P.n_tc_tiles) k_eeq_tc_tiles<<<P.n_tc_tiles, 256, 0, s>>>(V, B, P.tc_tiles.p);
+        if (P.cg_on) P.cg_launch(V, s);
+        if (!P.cg_on || P.nmol > 1) {   // Cholesky: of every molecule, or of those left over
+            EEQBatch B{P.roff.p, P.moff.p, P.border.p, P.bitems.p, P.nbitems, P.bnext.p, P.batch_smem_max, P.red2atom.p,
+                       P.anchor.p, P.qlist.p, P.nq, P.q0.p, P.M.p, P.bvec.p, P.info.p,
+                       P.batch_tc ? 1 : 0, P.M64.p, P.m64off.p, kRefineTol, P.refine.p, P.cg_on ? 1 : 0};
+            if (P.batch_tc) {
+                CK(cudaMemsetAsync(P.refine.p, 0, sizeof(int), s));
+                if (P.n_tc_tiles) k_eeq_tc_tiles<<<P.n_tc_tiles, 256, 0, s>>>(V, B, P.tc_tiles.p);
+            }
+            k_eeq_batch<<<P.batch_grid, 512, P.batch_smem, s>>>(V, B);
         }
-        k_eeq_batch<<<P.batch_grid, 512, P.batch_smem, s>>>(V, B);
         side_after();
     }
     const double* ysol = P.bvec.p;
