@@ -308,14 +308,12 @@ struct View {
     const double* c4;         // (3 szr^2)^(1/4): the product of two is sqrt(r4r2) of the pair
     const double* hmax;       // 72 max alpeeq: beyond this r^2 every Coulomb pair is 1/r
     // per step
-    double* cnraw;
     double* cn;
     double* dlog;
     double* wp;               // n*Rp current weights
     double* hdgp;             // n*Rp half contraction of the weights' CN derivative
     double* q;
     double* dEdcn;
-    double* v;
     double* grad;
     double* E;                // nmol*16 term energies
     int* status;              // nmol
@@ -328,9 +326,6 @@ struct View {
     int exact;                // drop the D4 dC6/dCN term
     double* cfar;             // n: potential of the Coulomb pairs beyond 100 bohr, or null
     const double* u;          // n: EEQ charge response, or null
-    // axis-aligned boxes of the runs of 32 consecutive atoms (current geometry)
-    const double4* boxlo;
-    const double4* boxhi;
     // periodic cell: the CN, bond, angle, HB, XB, repulsion, Coulomb and D4 pair distances
     // take the minimum image; torsions, inversions, ATM, BATM and the EEQ matrix do not
     Cell cell;

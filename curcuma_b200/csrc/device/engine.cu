@@ -290,7 +290,7 @@ struct Engine::Impl {
     // D4 pairs, when split from the Coulomb pairs, on a stream of their own beside the side
     // terms (GFNFF_D4_STREAM=0: before them on the side stream)
     cudaStream_t side_d4 = nullptr;
-    cudaEvent_t ev_join_d4 = nullptr;
+    cudaEvent_t ev_join_d4 = nullptr, ev_alpb = nullptr, ev_join_alpb = nullptr;
     bool side_early = false;   // GFNFF_SIDE_EARLY=1: fork at the start of the evaluation
     cusolverDnHandle_t sol = nullptr;
     int n = 0, nfrag = 0, K = 0, nred = 0, nmol = 0, nsplit = 1;
@@ -298,10 +298,9 @@ struct Engine::Impl {
     // directions by rows (GFNFF_PAIRS=rows)
     DBuf<int4> coul_tiles[3], d4_tiles[3];   // tile lists of k_pairs_coul and k_pairs_d4 per variant
     int n_coul_tiles[3] = {0, 0, 0}, n_d4_tiles[3] = {0, 0, 0};
-    DBuf<double4> boxlo, boxhi;   // per run of kBoxAtoms atoms
-    // CN neighbour list (k_cn_nl, k_cn_chain_nl): pairs within 6 + kCnSkin bohr of the
+    // CN neighbour list (k_cn_d4, k_tail): pairs within 6 + kCnSkin bohr of the
     // reference geometry cnl_ref, CSR by atom; cnl_bad = 1 once an atom moved more than
-    // kCnSkin / 2 from it (GFNFF_CN_LIST=0: all-pairs kernels only)
+    // kCnSkin / 2 from it (GFNFF_CN_LIST=0: every evaluation scans the molecule)
     static constexpr double kCnSkin = 1.0;
     bool cnl_on = false;
     int* cnl_bad_host = nullptr;   // pinned; refreshed by fetch()
@@ -384,7 +383,6 @@ struct Engine::Impl {
         const int zero = 0;
         cnl_bad.upload(std::vector<int>{zero});
     }
-    bool box_cull = false;        // CN kernels skip far tiles (single molecules >= 8192 atoms)
     Cell cell{};                  // periodic cell (cell.on = 0: isolated system)
     bool pairs_sym = true;
     bool pairs_occ = false;   // GFNFF_PAIRS_OCC=1: the untuned choice of single molecules is the largest tile
@@ -570,7 +568,6 @@ struct Engine::Impl {
     }
     void cg_launch(const View& V, cudaStream_t s)
     {
-        CK(cudaMemsetAsync(cg_iters.p, 0, sizeof(int), s));
         CgArgs A = cg_args();
         if (cg_bins.size() > 1) CK(cudaEventRecord(cg_fork, s));
         for (size_t k = 0; k < cg_bins.size(); ++k) {
@@ -708,10 +705,10 @@ struct Engine::Impl {
     DBuf<double> r_al, r_ab;
     DBuf<unsigned char> r_kind;
     // per step
-    DBuf<double> cnraw, cn, dlog, wp, hdgp, q, dEdcn, v, grad, E, M, bvec, xyz_stage, msd;
+    DBuf<double> cn, dlog, wp, hdgp, q, dEdcn, grad, E, M, bvec, xyz_stage, msd;
     DBuf<double> gout, qout, cnout;
     DBuf<double> work;
-    DBuf<int> info, info2, status, ipiv, bad;
+    DBuf<int> info, info2, status, ipiv, bad, tail_done;
     int lwork = 0;
     int lda = 4;           // leading dimension of M (>= nred + 1, a multiple of 4; row nred holds b for k_chol)
     bool use_lu = false;   // reduced EEQ matrix not positive definite: pivoted LU instead
@@ -893,16 +890,14 @@ struct Engine::Impl {
         V.slot = slot.p; V.nref = nref.p; V.refcn = refcn.p;
         V.Rp = Rp; V.kof = kof.p; V.pshift = pshift.p; V.w0p = w0p.p; V.g0p = g0p.p; V.c6p = c6p.p;
         V.zeta = zeta.p; V.szr = szr.p; V.c4 = c4.p; V.hmax = hmax.p; V.msd = msd.p;
-        V.cnraw = cnraw.p; V.cn = cn.p; V.dlog = dlog.p; V.wp = wp.p; V.hdgp = hdgp.p;
-        V.q = q.p; V.dEdcn = dEdcn.p; V.v = v.p; V.grad = grad.p; V.E = E.p; V.status = status.p;
+        V.cn = cn.p; V.dlog = dlog.p; V.wp = wp.p; V.hdgp = hdgp.p;
+        V.q = q.p; V.dEdcn = dEdcn.p; V.grad = grad.p; V.E = E.p; V.status = status.p;
         V.brad = alpb_on ? ab.brad.p : nullptr;
         V.bdiag = alpb_on ? ab.bdiag.p : nullptr;
         V.keps = alpb_on ? ab.keps : 0.0;
         V.exact = opt.exact_gradient ? 1 : 0;
         V.cfar = resp_on ? cfar.p : nullptr;
         V.u = resp_on ? ures.p : nullptr;
-        V.boxlo = box_cull ? boxlo.p : nullptr;
-        V.boxhi = box_cull ? boxhi.p : nullptr;
         V.cell = cell;
         return V;
     }
@@ -930,6 +925,8 @@ Engine::Engine(const EngineOptions& opt) : p_(new Impl)
         if (!(ds && !std::strcmp(ds, "0"))) {
             CK(cudaStreamCreateWithPriority(&p_->side_d4, cudaStreamNonBlocking, lo));
             CK(cudaEventCreateWithFlags(&p_->ev_join_d4, cudaEventDisableTiming));
+            CK(cudaEventCreateWithFlags(&p_->ev_alpb, cudaEventDisableTiming));
+            CK(cudaEventCreateWithFlags(&p_->ev_join_alpb, cudaEventDisableTiming));
         }
     }
     CS(cusolverDnCreate(&p_->sol));
@@ -967,7 +964,7 @@ Engine::~Engine()
         if (e) cudaEventDestroy(e);
     if (p_->sol) cusolverDnDestroy(p_->sol);
     if (p_->cnl_bad_host) cudaFreeHost(p_->cnl_bad_host);
-    for (cudaEvent_t e : {p_->ev_fork0, p_->ev_fork1, p_->ev_join, p_->ev_join_d4})
+    for (cudaEvent_t e : {p_->ev_fork0, p_->ev_fork1, p_->ev_join, p_->ev_join_d4, p_->ev_alpb, p_->ev_join_alpb})
         if (e) cudaEventDestroy(e);
     for (cudaStream_t st : p_->cg_streams) cudaStreamDestroy(st);
     for (cudaEvent_t e : p_->cg_done) cudaEventDestroy(e);
@@ -1259,10 +1256,6 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
             P.n_coul_tiles[v] = (int)c.size();
             P.n_d4_tiles[v] = (int)d.size();
         }
-        P.boxlo.alloc((n + kBoxAtoms - 1) / kBoxAtoms);
-        P.boxhi.alloc((n + kBoxAtoms - 1) / kBoxAtoms);
-        // box tests compare plain coordinates: off in a periodic cell
-        P.box_cull = nm == 1 && n >= 8192 && !P.cell.on;
         const char* pe = std::getenv("GFNFF_PAIRS");
         P.pairs_sym = !(pe && !std::strcmp(pe, "rows"));
         const char* po = std::getenv("GFNFF_PAIRS_OCC");
@@ -1667,7 +1660,7 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
         P.x_a.upload(xa); P.x_x.upload(xx); P.x_b.upload(xb); P.x_pre.upload(xpre); P.x_rv.upload(xrv);
     }
     // ---- per-step buffers ----
-    P.cnraw.alloc(n); P.cn.alloc(n); P.dlog.alloc(n); 
+    P.cn.alloc(n); P.dlog.alloc(n); 
     P.wp.upload(std::vector<double>((size_t)prows * Rp, 0.0));     // zero outside each atom's element
     P.hdgp.upload(std::vector<double>((size_t)prows * Rp, 0.0));   // and in the gaps between molecules
     P.etot.alloc(nm);
@@ -1686,7 +1679,7 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
             P.cfar.alloc(n); P.ures.alloc(n); P.bres.alloc(P.nred); P.xres.alloc(P.nred); P.info3.alloc(1);
         }
     }
-    P.q.alloc(n); P.dEdcn.alloc(n); P.v.alloc(n); P.grad.alloc(3 * (size_t)n); P.E.alloc(16 * (size_t)nm);
+    P.tail_done.upload(std::vector<int>{0}); P.q.alloc(n); P.dEdcn.alloc(n); P.grad.alloc(3 * (size_t)n); P.E.alloc(16 * (size_t)nm);
     P.gout.alloc(3 * (size_t)n); P.qout.alloc(n); P.cnout.alloc(n);
     P.lda = (P.nred + 4) & ~3;   // >= nred + 1, a multiple of 4: 16-byte aligned FP32 and FP64 columns
     P.M.alloc((size_t)std::max<long long>(1, nm == 1 ? (long long)P.lda * P.nred : P.msize));
@@ -2290,9 +2283,11 @@ void Engine::launch_positions(const double* d_xyz, bool bohr)
     Impl& P = *p_;
     P.mark(0);
     CK(cudaMemsetAsync(P.msd.p, 0, 3 * sizeof(double), P.stream));
+    StepZero Z{P.grad.p, P.dEdcn.p, P.resp_on ? P.cfar.p : nullptr, P.E.p, 16 * P.nmol, P.bad.p, P.nmol,
+               {P.tail_done.p, P.cg_iters.p, P.bnext.p, P.refine.p}};
     k_positions<<<nblk(P.n), kBlock, 0, P.stream>>>(P.n, P.perm.p, d_xyz, bohr ? 1.0 : kAngToBohr, P.pos.p,
                                                    P.hbref.p, P.msd.p, P.cnl_on ? P.cnl_ref.p : nullptr,
-                                                   0.25 * Impl::kCnSkin * Impl::kCnSkin, P.cnl_bad.p, P.toporef.p, P.pos0.p);
+                                                   0.25 * Impl::kCnSkin * Impl::kCnSkin, P.cnl_bad.p, P.toporef.p, P.pos0.p, Z);
 }
 
 // everything after the positions, reading and writing engine buffers only, so that it
@@ -2308,16 +2303,10 @@ void Engine::launch_body()
     // everywhere else (per-pair float<->double conversions cost more than FP32 saves in
     // the pair and CN-chain kernels) and in every accumulation
     const bool mixed = P.opt.precision == 1;
-    CK(cudaMemsetAsync(P.grad.p, 0, 3 * (size_t)n * sizeof(double), s));
-    CK(cudaMemsetAsync(P.dEdcn.p, 0, (size_t)n * sizeof(double), s));
-    CK(cudaMemsetAsync(P.cnraw.p, 0, (size_t)n * sizeof(double), s));
-    CK(cudaMemsetAsync(P.E.p, 0, 16 * (size_t)P.nmol * sizeof(double), s));
-    CK(cudaMemsetAsync(P.bad.p, 0, (size_t)P.nmol * sizeof(int), s));
-    if (P.resp_on) CK(cudaMemsetAsync(P.cfar.p, 0, (size_t)n * sizeof(double), s));
     // terms without a charge dependence: on the side stream when forking, else in phase order
     const bool fork = P.side && !P.timing;
     cudaStream_t s2 = fork ? P.side : s;
-    auto hb_rep_terms = [&]() {
+    auto hb_terms = [&]() {
     if (P.nhb) {
         HBSoA H{P.nhb, P.h_rec.p, P.h_qh.p, P.h_qa.p, P.h_bas.p, P.h_aci.p, P.h_rvdw.p, P.h_zlp.p,
                 P.h_pc.p, P.h_nfl.p, P.h_adjo.p, P.h_adj.p};
@@ -2330,23 +2319,28 @@ void Engine::launch_body()
             if (P.nhb > split) k_hbonds<float><<<nblk(P.nhb - split), kBlock, 0, s2>>>(V, H, split, P.nhb);
         }
     }
-    if (P.nxb) k_xbonds<<<nblk(P.nxb), kBlock, 0, s2>>>(V, XBSoA{P.nxb, P.x_a.p, P.x_x.p, P.x_b.p, P.x_pre.p, P.x_rv.p});
-    P.mark(8);
-    k_repulsion<double><<<nblk((long)n * 32), kBlock, 0, s2>>>(V, P.r_off.p, P.r_j.p, P.r_al.p, P.r_ab.p, P.r_kind.p);
-    P.mark(9);
+    };
+    // repulsion (warp per atom) and bonds (warp per bond), then the terms of a thread each
+    auto rep_bond_terms = [&](cudaStream_t st) {
+        k_repulsion<double><<<nblk((long)n * 32), kBlock, 0, st>>>(V, P.r_off.p, P.r_j.p, P.r_al.p, P.r_ab.p, P.r_kind.p);
+        if (!P.nb) return;
+        const BondSoA B{P.nb, P.b_i.p, P.b_j.p, P.b_h.p, P.b_off.p, P.b_hb.p, P.b_fc.p, P.b_al.p,
+                        P.b_r0i.p, P.b_r0j.p, P.b_cki.p, P.b_ckj.p, P.b_sh.p, P.b_ff.p};
+        k_bonds<<<nblk((long)P.nb * 32), kBlock, 0, st>>>(V, B);
     };
     auto bonded_terms = [&]() {
-    if (P.nb) {
-        BondSoA B{P.nb, P.b_i.p, P.b_j.p, P.b_h.p, P.b_off.p, P.b_hb.p, P.b_fc.p, P.b_al.p,
-                  P.b_r0i.p, P.b_r0j.p, P.b_cki.p, P.b_ckj.p, P.b_sh.p, P.b_ff.p};
-        k_bonds<<<nblk((long)P.nb * 32), kBlock, 0, s2>>>(V, B);
-    }
-    if (P.na) k_angles<<<nblk(P.na), kBlock, 0, s2>>>(V, AngleSoA{P.na, P.a_i.p, P.a_j.p, P.a_k.p, P.a_fc.p, P.a_th.p});
-    if (P.nt) k_torsions<<<nblk(P.nt), kBlock, 0, s2>>>(V, TorsSoA{P.nt, P.t_i.p, P.t_j.p, P.t_k.p, P.t_l.p, P.t_V.p, P.t_n.p, P.t_p.p}, 0);
-    if (P.ns) k_torsions<<<nblk(P.ns), kBlock, 0, s2>>>(V, TorsSoA{P.ns, P.s_i.p, P.s_j.p, P.s_k.p, P.s_l.p, P.s_e.p, nullptr, nullptr}, 1);
-    if (P.ninv) k_inversions<<<nblk(P.ninv), kBlock, 0, s2>>>(V, InvSoA{P.ninv, P.v_i.p, P.v_j.p, P.v_k.p, P.v_l.p, P.v_t.p, P.v_fc.p, P.v_om.p});
-    if (P.natm) k_atm<<<nblk(P.natm), kBlock, 0, s2>>>(V, TripSoA{P.natm, P.at_i.p, P.at_j.p, P.at_k.p, P.at_c9.p, P.at_r0ij.p, P.at_r0ik.p, P.at_r0jk.p, P.at_sc.p});
-    if (P.nbatm) k_batm<<<nblk(P.nbatm), kBlock, 0, s2>>>(V, TripSoA{P.nbatm, P.ba_i.p, P.ba_j.p, P.ba_k.p, P.ba_c9.p, nullptr, nullptr, nullptr, nullptr});
+        TermArgs A{{P.nbatm, P.ba_i.p, P.ba_j.p, P.ba_k.p, P.ba_c9.p, nullptr, nullptr, nullptr, nullptr},
+                   {P.natm, P.at_i.p, P.at_j.p, P.at_k.p, P.at_c9.p, P.at_r0ij.p, P.at_r0ik.p, P.at_r0jk.p, P.at_sc.p},
+                   {P.nt, P.t_i.p, P.t_j.p, P.t_k.p, P.t_l.p, P.t_V.p, P.t_n.p, P.t_p.p},
+                   {P.ns, P.s_i.p, P.s_j.p, P.s_k.p, P.s_l.p, P.s_e.p, nullptr, nullptr},
+                   {P.na, P.a_i.p, P.a_j.p, P.a_k.p, P.a_fc.p, P.a_th.p},
+                   {P.ninv, P.v_i.p, P.v_j.p, P.v_k.p, P.v_l.p, P.v_t.p, P.v_fc.p, P.v_om.p},
+                   {P.nxb, P.x_a.p, P.x_x.p, P.x_b.p, P.x_pre.p, P.x_rv.p},
+                   {}};
+        const int blocks[7] = {nblk(P.nbatm), nblk(P.nt), nblk(P.na), nblk(P.ninv), nblk(P.ns), nblk(P.natm), nblk(P.nxb)};
+        int end = 0;
+        for (int k = 0; k < 7; ++k) A.end[k] = end += blocks[k];
+        if (end) k_terms<<<end, kBlock, 0, s2>>>(V, A);
     };
     // The side terms fork right before the EEQ solve and are issued after the solver's
     // launch: the latency-bound cooperative PCG takes its SM slots first and the side
@@ -2372,37 +2366,40 @@ void Engine::launch_body()
         if (!split) return;
         if (sd != s2) CK(cudaStreamWaitEvent(sd, P.ev_fork1, 0));
         pairs_sym(std::integral_constant<int, kPairD4>{}, sd);
-        if (sd != s2) CK(cudaEventRecord(P.ev_join_d4, sd));
+    };
+    // with a stream of its own for the D4 pairs, repulsion and bonds follow them there
+    auto d4_rest = [&]() {
+        rep_bond_terms(sd);
+        if (split && sd != s2) CK(cudaEventRecord(P.ev_join_d4, sd));
     };
     const bool early = fork && P.side_early;
     if (early) {
         CK(cudaEventRecord(P.ev_fork0, s));
         CK(cudaStreamWaitEvent(s2, P.ev_fork0, 0));
-        hb_rep_terms();
+        hb_terms();
     }
     auto side_after = [&]() {
         if (!fork || early) return;
         CK(cudaStreamWaitEvent(s2, P.ev_fork1, 0));
         d4_pairs();
-        hb_rep_terms();
+        hb_terms();
+        d4_rest();
         bonded_terms();
         CK(cudaEventRecord(P.ev_join, s2));
     };
     P.mark(1);
-    if (P.box_cull) k_boxes<<<nblk(n, kTile), kTile, 0, s>>>(n, P.pos.p, P.boxlo.p, P.boxhi.p);
-    if (P.cnl_on) {
-        (mixed ? k_cn_nl<float> : k_cn_nl<double>)<<<nblk((long)n * 32), kBlock, 0, s>>>(V, P.cnl_off.p, P.cnl_j.p,
-                                                                                         P.cnl_bad.p);
-        (mixed ? k_cn<float> : k_cn<double>)<<<tgrid, kTile, 0, s>>>(V, P.nsplit, P.cnl_bad.p);
-    } else {
-        (mixed ? k_cn<float> : k_cn<double>)<<<tgrid, kTile, 0, s>>>(V, P.nsplit, nullptr);
-    }
+    const int* cn_off = P.cnl_on ? P.cnl_off.p : nullptr;
+    const unsigned watoms = nblk((long)n * 32);
+    if (V.cell.on)
+        (mixed ? k_cn_d4<float, true> : k_cn_d4<double, true>)<<<watoms, kBlock, 0, s>>>(V, nullptr, nullptr, nullptr);
+    else
+        (mixed ? k_cn_d4<float, false> : k_cn_d4<double, false>)<<<watoms, kBlock, 0, s>>>(V, cn_off, P.cnl_j.p, P.cnl_bad.p);
     P.mark(2);
-    k_d4_weights<<<nblk((long)n * 8), kBlock, 0, s>>>(V);
     if (early) {
         CK(cudaEventRecord(P.ev_fork1, s));
         CK(cudaStreamWaitEvent(s2, P.ev_fork1, 0));
         d4_pairs();
+        d4_rest();
         bonded_terms();
         CK(cudaEventRecord(P.ev_join, s2));
     }
@@ -2452,17 +2449,13 @@ void Engine::launch_body()
     } else {
         P.mark(4);
         P.mark(5);
-        CK(cudaMemsetAsync(P.bnext.p, 0, sizeof(int), s));
         if (fork && !early) CK(cudaEventRecord(P.ev_fork1, s));   // single molecule, batched solver
         if (P.cg_on) P.cg_launch(V, s);
         if (!P.cg_on || P.nmol > 1) {   // Cholesky: of every molecule, or of those left over
             EEQBatch B{P.roff.p, P.moff.p, P.border.p, P.bitems.p, P.nbitems, P.bnext.p, P.batch_smem_max, P.red2atom.p,
                        P.anchor.p, P.qlist.p, P.nq, P.q0.p, P.M.p, P.bvec.p, P.info.p,
                        P.batch_tc ? 1 : 0, P.M64.p, P.m64off.p, kRefineTol, P.refine.p, P.cg_on ? 1 : 0};
-            if (P.batch_tc) {
-                CK(cudaMemsetAsync(P.refine.p, 0, sizeof(int), s));
-                if (P.n_tc_tiles) k_eeq_tc_tiles<<<P.n_tc_tiles, 256, 0, s>>>(V, B, P.tc_tiles.p);
-            }
+            if (P.batch_tc && P.n_tc_tiles) k_eeq_tc_tiles<<<P.n_tc_tiles, 256, 0, s>>>(V, B, P.tc_tiles.p);
             k_eeq_batch<<<P.batch_grid, 512, P.batch_smem, s>>>(V, B);
         }
         side_after();
@@ -2476,7 +2469,20 @@ void Engine::launch_body()
     if (!fork) {
         bonded_terms();
         P.mark(7);
-        hb_rep_terms();
+        hb_terms();
+        P.mark(8);
+        rep_bond_terms(s2);
+        P.mark(9);
+    }
+    // solvation energy and gradient at the solved charges; beside the pairs on the D4 stream, which
+    // is free once its pairs are done
+    const bool alpb_side = P.alpb_on && fork && P.side_d4;
+    if (P.alpb_on && !alpb_side) P.alpb_post(s);
+    if (alpb_side) {
+        CK(cudaEventRecord(P.ev_alpb, s));
+        CK(cudaStreamWaitEvent(P.side_d4, P.ev_alpb, 0));
+        P.alpb_post(P.side_d4);
+        CK(cudaEventRecord(P.ev_join_alpb, P.side_d4));
     }
     if (P.pairs_sym) {
         if (!split) pairs_sym(std::integral_constant<int, kPairD4>{}, s);
@@ -2501,19 +2507,12 @@ void Engine::launch_body()
     }
     if (fork) CK(cudaStreamWaitEvent(s, P.ev_join, 0));
     if (split && sd != s2) CK(cudaStreamWaitEvent(s, P.ev_join_d4, 0));
+    if (alpb_side) CK(cudaStreamWaitEvent(s, P.ev_join_alpb, 0));
     P.mark(10);
-    k_post<<<nblk(n), kBlock, 0, s>>>(V);
-    if (P.cnl_on) {
-        k_cn_chain_nl<<<nblk((long)n * 32), kBlock, 0, s>>>(V, P.cnl_off.p, P.cnl_j.p, P.cnl_bad.p);
-        k_cn_chain<double><<<tgrid, kTile, 0, s>>>(V, P.nsplit, P.cnl_bad.p);
-    } else {
-        k_cn_chain<double><<<tgrid, kTile, 0, s>>>(V, P.nsplit, nullptr);
-    }
-    if (P.alpb_on) P.alpb_post(s);   // solvation energy and gradient at the solved charges
     P.mark(11);
-    k_outputs<<<nblk(n), kBlock, 0, s>>>(V, P.gout.p, P.qout.p, P.cnout.p, P.bad.p);
-    k_finish<<<nblk(P.nmol), kBlock, 0, s>>>(V, (P.nred > 0 || P.nmol > 1) ? P.info.p : nullptr, P.bad.p, P.e0.p,
-                                             P.etot.p);
+    const TailArgs T{V.cell.on ? nullptr : cn_off, P.cnl_j.p, P.cnl_bad.p, P.gout.p, P.qout.p, P.cnout.p, P.bad.p,
+                     (P.nred > 0 || P.nmol > 1) ? P.info.p : nullptr, P.e0.p, P.etot.p, (unsigned*)P.tail_done.p};
+    (V.cell.on ? k_tail<true> : k_tail<false>)<<<watoms, kBlock, 0, s>>>(V, T);
 }
 
 const double* Engine::d_terms() const { return p_->E.p; }

@@ -105,9 +105,9 @@ struct AngleSoA {
 };
 
 // angles with distance damping (ff_workspace_gfnff.cpp:187-280)
-__global__ void k_angles(View V, AngleSoA A)
+__device__ void angle_term(const View& V, int block, const AngleSoA& A)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = block * blockDim.x + threadIdx.x;
     double et = 0.0;
     if (t < A.n) {
         const int ia = A.i[t], ja = A.j[t], ka = A.k[t];
@@ -152,9 +152,9 @@ struct TorsSoA {
 
 // torsions + extra torsions (ff_workspace_gfnff.cpp:282-487), triple-bond torsions
 // (:611-653) when storsion = true
-__global__ void k_torsions(View V, TorsSoA T, int storsion)
+__device__ void torsion_term(const View& V, int block, const TorsSoA& T, int storsion)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = block * blockDim.x + threadIdx.x;
     double et = 0.0;
     if (t < T.n) {
         const int a = T.i[t], b = T.j[t], c = T.k[t], d = T.l[t];
@@ -204,9 +204,9 @@ struct InvSoA {
 };
 
 // inversions (ff_workspace_gfnff.cpp:489-609)
-__global__ void k_inversions(View V, InvSoA I)
+__device__ void inversion_term(const View& V, int block, const InvSoA& I)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = block * blockDim.x + threadIdx.x;
     double etot = 0.0;
     if (t < I.n) {
         const int a = I.i[t], b = I.j[t], c = I.k[t], d = I.l[t];
@@ -256,9 +256,9 @@ struct TripSoA {
 };
 
 // D4 ATM over bonded triplets (ff_workspace_gfnff.cpp:1526-1663)
-__global__ void k_atm(View V, TripSoA A)
+__device__ void atm_term(const View& V, int block, const TripSoA& A)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = block * blockDim.x + threadIdx.x;
     double et = 0.0;
     if (t < A.n) {
         const int a = A.i[t], b = A.j[t], c = A.k[t];
@@ -297,9 +297,9 @@ __global__ void k_atm(View V, TripSoA A)
 }
 
 // bonded ATM with the Phase-1 charge factors folded into c9 (ff_workspace_gfnff.cpp:1665-1739)
-__global__ void k_batm(View V, TripSoA A)
+__device__ void batm_term(const View& V, int block, const TripSoA& A)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = block * blockDim.x + threadIdx.x;
     double et = 0.0;
     if (t < A.n) {
         const int a = A.i[t], b = A.j[t], c = A.k[t];
@@ -651,9 +651,9 @@ struct XBSoA {
 };
 
 // halogen bonds (ff_workspace_gfnff.cpp:1411-1524); pre = -Q_B * acidity_X * Q_X
-__global__ void k_xbonds(View V, XBSoA S)
+__device__ void xbond_term(const View& V, int block, const XBSoA& S)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = block * blockDim.x + threadIdx.x;
     double etot = 0.0;
     if (t < S.n) {
         const double XB_BACUT = 70.0, XB_SCUT = 5.0, ALP = 6.0, LC = 70.0;

@@ -36,14 +36,28 @@ __device__ __forceinline__ void tile_range(const View& V, int i0, int nsplit, in
 // geometry topo_ref of the last topology (gfnff_method.cpp:1021-1031), as the bits of a
 // non-negative double (which order like the integers); msd[2] the largest |coordinate change|
 // since the set-up geometry pos0 (all atoms of a batch)
+// Also clears what the evaluation adds into (Z): a memset node each cost more than the writes.
+struct StepZero {
+    double *grad, *dEdcn, *cfar, *E;   // 3n, n, n (or null), nE
+    int nE;
+    int* bad;                          // nmol
+    int nmol;
+    int* words[4];                     // single counters (or null)
+};
 __global__ void k_positions(int n, const int* __restrict__ perm, const double* __restrict__ xyz, double scale,
                             double4* pos, const double4* __restrict__ ref, double* msd,
                             const double4* __restrict__ nl_ref, double nl_lim2, int* nl_bad,
-                            const double4* __restrict__ topo_ref, const double4* __restrict__ pos0)
+                            const double4* __restrict__ topo_ref, const double4* __restrict__ pos0, StepZero Z)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     double s = 0.0, dmax = 0.0, d0max = 0.0;
+    for (int k = i; k < Z.nE; k += gridDim.x * blockDim.x) Z.E[k] = 0.0;
+    for (int k = i; k < Z.nmol; k += gridDim.x * blockDim.x) Z.bad[k] = 0;
+    if (i < 4 && Z.words[i]) *Z.words[i] = 0;
     if (i < n) {
+        Z.grad[3 * i] = Z.grad[3 * i + 1] = Z.grad[3 * i + 2] = 0.0;
+        Z.dEdcn[i] = 0.0;
+        if (Z.cfar) Z.cfar[i] = 0.0;
         const int o = perm[i];
         const double x = xyz[3 * o] * scale, y = xyz[3 * o + 1] * scale, z = xyz[3 * o + 2] * scale;
         pos[i] = make_double4(x, y, z, 0.0);
@@ -72,62 +86,6 @@ __global__ void k_positions(int n, const int* __restrict__ perm, const double* _
     block_add(s, msd);
 }
 
-// ------------------------------------------------------------------------------------
-// atom boxes: min/max corner of every run of 32 consecutive atoms.  Atoms are in Morton
-// order within a molecule, so a run is fairly compact in space and the short-range pair
-// kernels (CN, CN chain rule) skip partner tiles, and a warp partner runs of 32 atoms, whose
-// box is farther than the cutoff from its own (single molecules of 8192 atoms or more;
-// below that the tests cost more than they save, measured).  The box distance is a lower bound of every pair distance
-// in floating point too (min/max are exact, rounding is monotonic), so the skipped pairs
-// are exactly pairs the cutoff test rejects.
-// ------------------------------------------------------------------------------------
-constexpr int kBoxAtoms = 32;
-__global__ void __launch_bounds__(kTile) k_boxes(int n, const double4* __restrict__ pos, double4* lo, double4* hi)
-{
-    const int i = blockIdx.x * kTile + threadIdx.x;
-    const int b = i / kBoxAtoms;
-    if (b * kBoxAtoms >= n) return;   // whole warp beyond the atoms
-    const double4 p = pos[i < n ? i : b * kBoxAtoms];
-    double v[6] = {p.x, p.y, p.z, -p.x, -p.y, -p.z};   // minima of x and of -x
-#pragma unroll
-    for (int k = 0; k < 6; ++k)
-        for (int o = 16; o > 0; o >>= 1) v[k] = fmin(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
-    if ((threadIdx.x & 31) == 0) {
-        lo[b] = make_double4(v[0], v[1], v[2], 0.0);
-        hi[b] = make_double4(-v[3], -v[4], -v[5], 0.0);
-    }
-}
-
-// box of the atoms [a, b) (b > a), as the union of the 32-atom boxes covering it
-__device__ __forceinline__ void range_box(const View& V, int a, int b, double4& l, double4& h)
-{
-    l = V.boxlo[a / kBoxAtoms];
-    h = V.boxhi[a / kBoxAtoms];
-    for (int k = a / kBoxAtoms + 1; k <= (b - 1) / kBoxAtoms; ++k) {
-        const double4 l2 = V.boxlo[k], h2 = V.boxhi[k];
-        l = make_double4(fmin(l.x, l2.x), fmin(l.y, l2.y), fmin(l.z, l2.z), 0.0);
-        h = make_double4(fmax(h.x, h2.x), fmax(h.y, h2.y), fmax(h.z, h2.z), 0.0);
-    }
-}
-
-__device__ __forceinline__ bool boxes_far(double4 il, double4 ih, double4 jl, double4 jh, double cut2)
-{
-    const double dx = fmax(0.0, fmax(jl.x - ih.x, il.x - jh.x));
-    const double dy = fmax(0.0, fmax(jl.y - ih.y, il.y - jh.y));
-    const double dz = fmax(0.0, fmax(jl.z - ih.z, il.z - jh.z));
-    return dx * dx + dy * dy + dz * dz >= cut2;
-}
-
-// true when every atom of [j0, j0 + cnt) is at least sqrt(cut2) from every atom of
-// [i0, i0 + ni)
-__device__ __forceinline__ bool ranges_far(const View& V, int i0, int ni, int j0, int cnt, double cut2)
-{
-    double4 il, ih, jl, jh;
-    range_box(V, i0, i0 + ni, il, ih);
-    range_box(V, j0, j0 + cnt, jl, jh);
-    return boxes_far(il, ih, jl, jh, cut2);
-}
-
 // One counting term 0.5 (1 + erf(kn (r - rc) / rc)), kn = -7.5, of the GFN-FF CN
 // (cn_calculator.cpp:367-428); d2 = r^2, rc = the pair's covalent radius sum (bohr).  FP64:
 // as written.  FP32 (mixed form): the argument in FP64, then the identity 0.5 (1 + erf(z)) =
@@ -148,67 +106,64 @@ __device__ __forceinline__ double cn_count(double d2, double rc)
 }
 
 // ------------------------------------------------------------------------------------
-// coordination numbers: erf counting over partners closer than 6 bohr
-// (cn_calculator.cpp:367-428); the log-squash is applied in k_d4_weights
+// Coordination numbers (erf counting over partners closer than 6 bohr, cn_calculator.cpp:367-428),
+// their log-squash (cnmax = 4.4) and its derivative, D4 Gaussian weights (wf = 4) and the half
+// contraction of their derivative with the reference C6 (d4param_generator.cpp:1079-1290,
+// :1692-1740): one warp per atom, one launch (CN by list, CN by all pairs when the list is stale,
+// and the weights were three).
+//
+// The partners come from a Verlet list (pairs within 6 + 1 bohr at the list's reference geometry,
+// same molecule, CSR by atom, both directions), valid while no atom moved more than half the
+// 1-bohr skin (*nl_bad, checked in k_positions at every evaluation).  Without a valid list the
+// warp scans its molecule, 32 atoms a step: 2 x 3 us on 194 atoms where a block per 128 atoms and
+// partner tiles in shared memory took 41 (CN) and 48 us (chain rule).
+//
+// The weights: lane r of every eight holds reference r (7 at most), so the exponentials of an atom
+// run side by side, and the lanes then share the packed references.
 // ------------------------------------------------------------------------------------
-template <class R>
-__global__ void __launch_bounds__(kTile) k_cn(View V, int nsplit, const int* nl_bad)
+template <bool CELL, class F>
+__device__ __forceinline__ void cn_partners(const View& V, int i, const double4& pi, const int* off, const int* nbr,
+                                            const int* nl_bad, F f)
 {
-    if (nl_bad && *nl_bad == 0) return;   // the neighbour-list kernel does the work
-    __shared__ double sx[kTile], sy[kTile], sz[kTile], sr[kTile];
-    const int i0 = blockIdx.x * kTile, i = i0 + threadIdx.x;
-    int jb, je;
-    tile_range(V, i0, nsplit, jb, je);
-    const bool act = i < V.n;
-    const double4 pi = act ? V.pos[i] : make_double4(0.0, 0.0, 0.0, 0.0);
-    const double ri = act ? V.rcov_cn[i] : 0.0;
-    const int2 rg = act ? V.jr[i] : make_int2(0, 0);
-    double s = 0.0;
-    const int ni = min(kTile, V.n - i0);
-    const int w0 = i0 + (threadIdx.x & ~31), nw = max(0, min(32, V.n - w0));   // this warp's atoms
-    for (int t0 = jb; t0 < je; t0 += kTile) {
-        const int cnt = min(kTile, je - t0);
-        if (V.boxlo && ranges_far(V, i0, ni, t0, cnt, 36.0)) continue;   // uniform in the block
-        __syncthreads();
-        const int jl = t0 + threadIdx.x;
-        if (jl < je) {
-            const double4 p = V.pos[jl];
-            sx[threadIdx.x] = p.x; sy[threadIdx.x] = p.y; sz[threadIdx.x] = p.z;
-            sr[threadIdx.x] = V.rcov_cn[jl];
+    const int lane = threadIdx.x & 31;
+    if (off && *nl_bad == 0) {
+        for (int p = off[i] + lane; p < off[i + 1]; p += 32) {
+            const int j = nbr[p];
+            const double4 pj = V.pos[j];
+            const double dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
+            const double d2 = dx * dx + dy * dy + dz * dz;
+            if (d2 < 36.0) f(j, dx, dy, dz, d2);
         }
-        __syncthreads();
-        if (!act) continue;
-        for (int js = 0; js < cnt; js += 32) {
-            const int jn = min(32, cnt - js);
-            if (V.boxlo && ranges_far(V, w0, nw, t0 + js, jn, 36.0)) continue;   // uniform in the warp
-            for (int jj = js; jj < js + jn; ++jj) {
-                double dx = pi.x - sx[jj], dy = pi.y - sy[jj], dz = pi.z - sz[jj];
-                if (V.cell.on) mic(V.cell, dx, dy, dz);
-                const double d2 = dx * dx + dy * dy + dz * dz;
-                const int j = t0 + jj;
-                if (!(d2 < 36.0) || j == i || j < rg.x || j >= rg.y) continue;
-                s += cn_count<R>(d2, ri + sr[jj]);
-            }
+    } else {
+        const int2 rg = V.jr[i];
+        for (int j = rg.x + lane; j < rg.y; j += 32) {
+            const double4 pj = V.pos[j];
+            double dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
+            if (CELL) mic(V.cell, dx, dy, dz);
+            const double d2 = dx * dx + dy * dy + dz * dz;
+            if (d2 < 36.0 && j != i) f(j, dx, dy, dz, d2);
         }
     }
-    if (act && s != 0.0) atomicAdd(V.cnraw + i, s);
 }
 
-// ------------------------------------------------------------------------------------
-// CN log-squash (cnmax = 4.4) and its derivative, D4 Gaussian weights (wf = 4) and the
-// half contraction with the reference C6 (d4param_generator.cpp:1079-1290, :1692-1740)
-// ------------------------------------------------------------------------------------
-// Eight lanes per atom: lane r holds reference r (7 at most), so the exponentials of an atom run
-// side by side, and the lanes then share the half contraction over the packed references (a
-// thread per atom took 14 us on 194 atoms and 24 us on 20,480: a chain of 7 exp and K 49 loads).
-__global__ void __launch_bounds__(kBlock) k_d4_weights(View V)
+template <class R, bool CELL>
+__global__ void __launch_bounds__(kBlock) k_cn_d4(View V, const int* __restrict__ off, const int* __restrict__ nbr,
+                                                 const int* nl_bad)
 {
     constexpr unsigned full = 0xffffffffu;
-    const int i0 = (blockIdx.x * kBlock + threadIdx.x) >> 3, r = threadIdx.x & 7;
-    const int i = min(i0, V.n - 1);   // whole warps stay: the lanes exchange values
-    const double cnmax = 4.4, s = V.cnraw[i];
+    const int i = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (i >= V.n) return;
+    const double4 pi = V.pos[i];
+    const double ri = V.rcov_cn[i];
+    double s = 0.0;
+    cn_partners<CELL>(V, i, pi, off, nbr, nl_bad, [&](int j, double, double, double, double d2) {
+        s += cn_count<R>(d2, ri + V.rcov_cn[j]);
+    });
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(full, s, o);
+    const double cnmax = 4.4;
     const double cn = log(1.0 + exp(cnmax)) - log(1.0 + exp(cnmax - s));
-    const int nr = V.nref[i];
+    const int nr = V.nref[i], r = lane & 7;
     double ex = 0.0, dex = 0.0;
     if (r < nr) {
         const double d = cn - V.refcn[i * 7 + r];
@@ -232,23 +187,22 @@ __global__ void __launch_bounds__(kBlock) k_d4_weights(View V)
         }
     }
     const double z = V.zeta[i];
-    const bool act = i0 < V.n;
-    if (act && r == 0) {
+    const int row = i + V.pshift[V.nmol == 1 ? 0 : V.mol[i]];
+    if (lane == 0) {
         V.cn[i] = cn;
         V.dlog[i] = exp(cnmax) / (exp(cnmax) + exp(s));
     }
-    const int row = i + V.pshift[V.nmol == 1 ? 0 : V.mol[i]];
-    if (act && r < nr) V.wp[pk(V.Rp, row, V.kof[i] + r)] = z * w;
+    if (lane < nr) V.wp[pk(V.Rp, row, V.kof[i] + lane)] = z * w;
     const double* C = V.c6p + (size_t)V.slot[i] * 7 * V.Rp;
     double dwa[7];
 #pragma unroll
-    for (int a = 0; a < 7; ++a) dwa[a] = __shfl_sync(full, dw, (threadIdx.x & 24) + a);
-    for (int k = r; k < V.Rp; k += 8) {
+    for (int a = 0; a < 7; ++a) dwa[a] = __shfl_sync(full, dw, a);
+    for (int k = lane; k < V.Rp; k += 32) {
         double dg = 0.0;
 #pragma unroll
         for (int a = 0; a < 7; ++a)
             if (a < nr) dg += dwa[a] * C[a * V.Rp + k];
-        if (act) V.hdgp[pk(V.Rp, row, k)] = z * dg;
+        V.hdgp[pk(V.Rp, row, k)] = z * dg;
     }
 }
 
@@ -310,6 +264,15 @@ __global__ void __launch_bounds__(kBlock) k_repulsion(View V, const int* off, co
 // plain form of the terms; k_pairs_coul and k_pairs_d4 (k_pairs.cuh) evaluate the same pairs once.  It is one of
 // the set-up tuner's variants ("rows").
 // ------------------------------------------------------------------------------------
+// Coulomb self term of atom i (ff_workspace.cpp:415-536)
+__device__ __forceinline__ double coulomb_self(const View& V, int i)
+{
+    const int2 rg = V.jr[i];
+    if (rg.y - rg.x < 2 || !(V.alpeeq[i] > 0.0)) return 0.0;
+    const double q = V.q[i], chi = V.chi_base[i] + V.cnf[i] * sqrt(fmax(V.cn[i], 0.0));
+    return -q * chi + 0.5 * q * q * V.adiag[i];
+}
+
 // one D4 pair: energy e, dE/dr / r in dedr, dE/dCN_i in dc (zeta folded into the operands)
 __device__ __forceinline__ void d4_pair(const View& V, double d2, int rowi, int kj, const double (*sw0)[kTile],
                                         const double (*sw)[kTile], int jj, int nr, double szi, double szj,
@@ -416,14 +379,14 @@ __global__ void __launch_bounds__(kTile) k_pairs(View V, int nsplit)
         if (cfar != 0.0) atomicAdd(V.cfar + i, cfar);
     }
     const int m = act ? V.mol[i] : -1;
-    eadd(V, 0.5 * ec, m, T_COUL);
+    eadd(V, 0.5 * ec + (act && blockIdx.y == 0 ? coulomb_self(V, i) : 0.0), m, T_COUL);
     eadd(V, 0.5 * ed, m, T_DISP);
 }
 
 // ------------------------------------------------------------------------------------
 // EEQ charge response (exact-gradient mode): with u = B M^-1 B^T w and w = dE/dq of the
 // Coulomb pairs cut at 100 bohr, the gradient gains -sum_ij u_i q_j dA_ij/dr over all
-// pairs (A is the uncut EEQ matrix) and u_i dx_i/dCN_i through the CN chain (k_post).
+// pairs (A is the uncut EEQ matrix) and u_i dx_i/dCN_i through the CN chain (k_tail).
 // ------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kTile) k_resp_pairs(View V, int nsplit)
 {
@@ -475,116 +438,88 @@ __global__ void __launch_bounds__(kTile) k_resp_pairs(View V, int nsplit)
 }
 
 // ------------------------------------------------------------------------------------
-// Coulomb self terms and the CN-chain weight u = dlogCN (dE/dCN - q cnf/(2 sqrt CN))
-// (ff_workspace.cpp:415-536)
+// The end of an evaluation, a warp per atom: the CN chain rule
+// grad_i += sum_j dS_ij/dr (v_i + v_j) (x_i - x_j)/r over the 6 bohr neighbours
+// (gfnff_method.cpp:5837-6260, forcefieldthread.h:80-109) with the chain weight
+// v = dlogCN (dE/dCN - q cnf/(2 sqrt CN)) (ff_workspace.cpp:415-536) formed where it is read, the
+// outputs in the caller's atom order, finiteness flags per molecule; the last block to finish
+// sums the totals and statuses of the molecules.  One launch for what were five (weights, chain
+// by list, chain by all pairs, outputs, totals); partners as in k_cn_d4.
 // ------------------------------------------------------------------------------------
-__global__ void k_post(View V)
+struct TailArgs {
+    const int *off, *nbr, *nl_bad;
+    double *gout, *qout, *cnout;
+    int* bad;
+    const int* eeq_info;
+    const double* e0;
+    double* etot;
+    unsigned* done;   // blocks finished; back to 0 at the end
+};
+
+__device__ __forceinline__ double chain_weight(const View& V, int i)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double e = 0.0;
+    const double q = V.q[i], cn = fmax(V.cn[i], 0.0);
+    // the EEQ charge response u adds u dx/dCN (exact-gradient mode)
+    const double qe = V.u ? q - V.u[i] : q;
+    return V.dlog[i] * (V.dEdcn[i] - qe * V.cnf[i] / (2.0 * sqrt(cn) + 1e-16));
+}
+
+template <bool CELL>
+__global__ void __launch_bounds__(kBlock) k_tail(View V, TailArgs T)
+{
+    __shared__ bool last;
+    const int i = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (i < V.n) {
-        const double q = V.q[i], cn = fmax(V.cn[i], 0.0);
-        const int2 rg = V.jr[i];
-        if (rg.y - rg.x >= 2 && V.alpeeq[i] > 0.0) {
-            const double chi = V.chi_base[i] + V.cnf[i] * sqrt(cn);
-            e = -q * chi + 0.5 * q * q * V.adiag[i];
-        }
-        // the EEQ charge response u adds u dx/dCN (exact-gradient mode)
-        const double qe = V.u ? q - V.u[i] : q;
-        V.v[i] = V.dlog[i] * (V.dEdcn[i] - qe * V.cnf[i] / (2.0 * sqrt(cn) + 1e-16));
-    }
-    eadd(V, e, i < V.n ? V.mol[i] : -1, T_COUL);
-}
-
-// CN chain rule: grad_i += sum_j dS_ij/dr (u_i + u_j) (x_i - x_j)/r over the 6 bohr
-// neighbours (gfnff_method.cpp:5837-6260, forcefieldthread.h:80-109)
-template <class R>
-__global__ void __launch_bounds__(kTile) k_cn_chain(View V, int nsplit, const int* nl_bad)
-{
-    if (nl_bad && *nl_bad == 0) return;   // the neighbour-list kernel does the work
-    __shared__ double sx[kTile], sy[kTile], sz[kTile], sr[kTile], su[kTile];
-    const int i0 = blockIdx.x * kTile, i = i0 + threadIdx.x;
-    int jb, je;
-    tile_range(V, i0, nsplit, jb, je);
-    const bool act = i < V.n;
-    const double4 pi = act ? V.pos[i] : make_double4(0.0, 0.0, 0.0, 0.0);
-    const double ri = act ? V.rcov_cn[i] : 0.0;
-    const double ui = act ? V.v[i] : 0.0;
-    const int2 rg = act ? V.jr[i] : make_int2(0, 0);
-    const double kn = -7.5, sqrtpi = 1.77245385091;
-    double gx = 0.0, gy = 0.0, gz = 0.0;
-    const int ni = min(kTile, V.n - i0);
-    const int w0 = i0 + (threadIdx.x & ~31), nw = max(0, min(32, V.n - w0));   // this warp's atoms
-    for (int t0 = jb; t0 < je; t0 += kTile) {
-        const int cnt = min(kTile, je - t0);
-        if (V.boxlo && ranges_far(V, i0, ni, t0, cnt, 36.0)) continue;   // uniform in the block
-        __syncthreads();
-        const int jl = t0 + threadIdx.x;
-        if (jl < je) {
-            const double4 p = V.pos[jl];
-            sx[threadIdx.x] = p.x; sy[threadIdx.x] = p.y; sz[threadIdx.x] = p.z;
-            sr[threadIdx.x] = V.rcov_cn[jl];
-            su[threadIdx.x] = V.v[jl];
-        }
-        __syncthreads();
-        if (!act) continue;
-        for (int js = 0; js < cnt; js += 32) {
-        const int jn = min(32, cnt - js);
-        if (V.boxlo && ranges_far(V, w0, nw, t0 + js, jn, 36.0)) continue;   // uniform in the warp
-        for (int jj = js; jj < js + jn; ++jj) {
-            double dx = sx[jj] - pi.x, dy = sy[jj] - pi.y, dz = sz[jj] - pi.z;
-            if (V.cell.on) mic(V.cell, dx, dy, dz);
-            const double d2 = dx * dx + dy * dy + dz * dz;
-            const int j = t0 + jj;
-            if (!(d2 < 36.0) || j == i || j < rg.x || j >= rg.y) continue;
-            const R r = sqrt((R)d2);
-            const R rs = (R)(ri + sr[jj]);
-            const R dr = (r - rs) / rs;
-            const R de = R(kn / sqrtpi) * exp(R(-kn * kn) * dr * dr) / rs;
-            const double f = -(double)(de / r) * (ui + su[jj]);
+        const double4 pi = V.pos[i];
+        const double ri = V.rcov_cn[i], vi = chain_weight(V, i);
+        const double kn = -7.5, sqrtpi = 1.77245385091;
+        double gx = 0.0, gy = 0.0, gz = 0.0;
+        cn_partners<CELL>(V, i, pi, T.off, T.nbr, T.nl_bad, [&](int j, double dx, double dy, double dz, double d2) {
+            const double r = sqrt(d2);
+            const double rs = ri + V.rcov_cn[j];
+            const double dr = (r - rs) / rs;
+            const double de = (kn / sqrtpi) * exp(-kn * kn * dr * dr) / rs;
+            const double f = -(de / r) * (vi + chain_weight(V, j));
             gx += f * dx; gy += f * dy; gz += f * dz;
+        });
+        for (int o = 16; o > 0; o >>= 1) {
+            gx += __shfl_down_sync(0xffffffffu, gx, o);
+            gy += __shfl_down_sync(0xffffffffu, gy, o);
+            gz += __shfl_down_sync(0xffffffffu, gz, o);
         }
+        if (lane == 0) {
+            const int o = V.perm[i];
+            gx += V.grad[3 * i];
+            gy += V.grad[3 * i + 1];
+            gz += V.grad[3 * i + 2];
+            T.gout[3 * o] = gx;
+            T.gout[3 * o + 1] = gy;
+            T.gout[3 * o + 2] = gz;
+            T.qout[o] = V.q[i];
+            T.cnout[o] = V.cn[i];
+            if (!isfinite(gx) || !isfinite(gy) || !isfinite(gz)) atomicOr(T.bad + V.mol[i], 1);
         }
     }
-    if (act) {
-        if (gx != 0.0) atomicAdd(V.grad + 3 * i, gx);
-        if (gy != 0.0) atomicAdd(V.grad + 3 * i + 1, gy);
-        if (gz != 0.0) atomicAdd(V.grad + 3 * i + 2, gz);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(T.done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    // per molecule: total energy, status (NOT_SPD from the EEQ factorisation, NONFINITE)
+    for (int m = threadIdx.x; m < V.nmol; m += blockDim.x) {
+        double tot = T.e0[m];
+        for (int t = 0; t < T_TOTAL; ++t) tot += V.E[16 * m + t];
+        V.E[16 * m + T_TOTAL] = tot;
+        T.etot[m] = tot;
+        int st = 0;
+        if (T.eeq_info && T.eeq_info[m] == 2) st = GFNFF_CUDA_ERROR;
+        else if (T.eeq_info && T.eeq_info[m] == 3) st = GFNFF_REFINE_NOT_CONVERGED;
+        else if (T.eeq_info && T.eeq_info[m] != 0) st = GFNFF_NOT_SPD;
+        else if (!isfinite(tot) || __ldcg(T.bad + m)) st = GFNFF_NONFINITE;
+        V.status[m] = st;
     }
-}
-
-// ------------------------------------------------------------------------------------
-// outputs in the caller's atom order, finiteness flags per molecule
-// ------------------------------------------------------------------------------------
-__global__ void k_outputs(View V, double* gout, double* qout, double* cnout, int* bad)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= V.n) return;
-    const int o = V.perm[i];
-    const double gx = V.grad[3 * i], gy = V.grad[3 * i + 1], gz = V.grad[3 * i + 2];
-    gout[3 * o] = gx;
-    gout[3 * o + 1] = gy;
-    gout[3 * o + 2] = gz;
-    qout[o] = V.q[i];
-    cnout[o] = V.cn[i];
-    if (!isfinite(gx) || !isfinite(gy) || !isfinite(gz)) atomicOr(bad + V.mol[i], 1);
-}
-
-// per molecule: total energy, status (NOT_SPD from the EEQ factorisation, NONFINITE)
-__global__ void k_finish(View V, const int* eeq_info, const int* bad, const double* e0, double* out_e)
-{
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= V.nmol) return;
-    double tot = e0[m];
-    for (int t = 0; t < T_TOTAL; ++t) tot += V.E[16 * m + t];
-    V.E[16 * m + T_TOTAL] = tot;
-    if (out_e) out_e[m] = tot;
-    int st = 0;
-    if (eeq_info && eeq_info[m] == 2) st = GFNFF_CUDA_ERROR;
-    else if (eeq_info && eeq_info[m] == 3) st = GFNFF_REFINE_NOT_CONVERGED;
-    else if (eeq_info && eeq_info[m] != 0) st = GFNFF_NOT_SPD;
-    else if (!isfinite(tot) || bad[m]) st = GFNFF_NONFINITE;
-    V.status[m] = st;
+    if (threadIdx.x == 0) *T.done = 0u;
 }
 
 // device enumeration of the D4 pair list at the setup geometry (topology check)
@@ -600,70 +535,30 @@ __global__ void k_disp_count(int n, const double4* pos0, const int2* jr, unsigne
     }
 }
 
-
 // ------------------------------------------------------------------------------------
-// CN and CN chain rule over a Verlet neighbour list (pairs within 6 + 1 bohr at the list's
-// reference geometry, same molecule; CSR by atom, both directions): a warp per atom, lanes
-// over its partners.  Valid while no atom moved more than half the 1-bohr skin (checked in
-// k_positions every evaluation); a stale list hands the work back to the all-pairs kernels
-// above in the same launch sequence, and the host rebuilds it.  Same arithmetic per pair as
-// k_cn / k_cn_chain; only the summation order of an atom's partners differs.
+// The terms with a thread per term (angles, torsions, inversions, three-body and halogen-bond
+// terms) in one launch: the blocks of the term lists follow one another (end[k]: first block past
+// list k).  As launches of their own (up to seven, 6-9 us each whatever their length) they were the
+// longest chain beside the charges on small molecules: 43 us with the repulsion for 26 atoms.
 // ------------------------------------------------------------------------------------
-template <class R>
-__global__ void __launch_bounds__(kBlock) k_cn_nl(View V, const int* __restrict__ off, const int* __restrict__ nbr,
-                                                 const int* nl_bad)
+struct TermArgs {
+    TripSoA BM, AT;
+    TorsSoA T, S;
+    AngleSoA A;
+    InvSoA I;
+    XBSoA X;
+    int end[7];
+};
+__global__ void __launch_bounds__(kBlock) k_terms(View V, TermArgs P)
 {
-    if (*nl_bad) return;
-    const int i = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (i >= V.n) return;
-    const double4 pi = V.pos[i];
-    const double ri = V.rcov_cn[i];
-    double s = 0.0;
-    for (int p = off[i] + lane; p < off[i + 1]; p += 32) {
-        const int j = nbr[p];
-        const double4 pj = V.pos[j];
-        const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-        const double d2 = dx * dx + dy * dy + dz * dz;
-        if (!(d2 < 36.0)) continue;
-        s += cn_count<R>(d2, ri + V.rcov_cn[j]);
-    }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0 && s != 0.0) atomicAdd(V.cnraw + i, s);
-}
-
-__global__ void __launch_bounds__(kBlock) k_cn_chain_nl(View V, const int* __restrict__ off,
-                                                       const int* __restrict__ nbr, const int* nl_bad)
-{
-    if (*nl_bad) return;
-    const int i = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (i >= V.n) return;
-    const double4 pi = V.pos[i];
-    const double ri = V.rcov_cn[i], ui = V.v[i];
-    const double kn = -7.5, sqrtpi = 1.77245385091;
-    double gx = 0.0, gy = 0.0, gz = 0.0;
-    for (int p = off[i] + lane; p < off[i + 1]; p += 32) {
-        const int j = nbr[p];
-        const double4 pj = V.pos[j];
-        const double dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
-        const double d2 = dx * dx + dy * dy + dz * dz;
-        if (!(d2 < 36.0)) continue;
-        const double r = sqrt(d2);
-        const double rs = ri + V.rcov_cn[j];
-        const double dr = (r - rs) / rs;
-        const double de = (kn / sqrtpi) * exp(-kn * kn * dr * dr) / rs;
-        const double f = -(de / r) * (ui + V.v[j]);
-        gx += f * dx; gy += f * dy; gz += f * dz;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        gx += __shfl_down_sync(0xffffffffu, gx, o);
-        gy += __shfl_down_sync(0xffffffffu, gy, o);
-        gz += __shfl_down_sync(0xffffffffu, gz, o);
-    }
-    if (lane == 0) {
-        if (gx != 0.0) atomicAdd(V.grad + 3 * i, gx);
-        if (gy != 0.0) atomicAdd(V.grad + 3 * i + 1, gy);
-        if (gz != 0.0) atomicAdd(V.grad + 3 * i + 2, gz);
-    }
+    const int b = blockIdx.x;
+    if (b < P.end[0]) batm_term(V, b, P.BM);
+    else if (b < P.end[1]) torsion_term(V, b - P.end[0], P.T, 0);
+    else if (b < P.end[2]) angle_term(V, b - P.end[1], P.A);
+    else if (b < P.end[3]) inversion_term(V, b - P.end[2], P.I);
+    else if (b < P.end[4]) torsion_term(V, b - P.end[3], P.S, 1);
+    else if (b < P.end[5]) atm_term(V, b - P.end[4], P.AT);
+    else xbond_term(V, b - P.end[5], P.X);
 }
 
 }  // namespace

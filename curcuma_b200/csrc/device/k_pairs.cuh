@@ -218,6 +218,8 @@ __global__ void __launch_bounds__(32 * WR, kPairWarps / WR) k_pairs_coul(View V,
             srow[warp][2][lane] = p.z;
             srow[warp][3][lane] = V.q[i];
         }
+        // the self terms of the rows, once: with the row block's first tile
+        if (j0 == tl.x && r0 + lane < iend) ec = coulomb_self(V, r0 + lane);
         __syncwarp();
         double ga[4][4];   // row sums
 #pragma unroll
