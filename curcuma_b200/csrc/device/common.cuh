@@ -310,6 +310,7 @@ struct View {
     // per step
     double* cn;
     double* dlog;
+    double* dxdcn;            // cnf / (2 sqrt CN): derivative of the EEQ right-hand side
     double* wp;               // n*Rp current weights
     double* hdgp;             // n*Rp half contraction of the weights' CN derivative
     double* q;

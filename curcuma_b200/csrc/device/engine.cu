@@ -705,7 +705,7 @@ struct Engine::Impl {
     DBuf<double> r_al, r_ab;
     DBuf<unsigned char> r_kind;
     // per step
-    DBuf<double> cn, dlog, wp, hdgp, q, dEdcn, grad, E, M, bvec, xyz_stage, msd;
+    DBuf<double> cn, dxdcn, dlog, wp, hdgp, q, dEdcn, grad, E, M, bvec, xyz_stage, msd;
     DBuf<double> gout, qout, cnout;
     DBuf<double> work;
     DBuf<int> info, info2, status, ipiv, bad, tail_done;
@@ -890,7 +890,7 @@ struct Engine::Impl {
         V.slot = slot.p; V.nref = nref.p; V.refcn = refcn.p;
         V.Rp = Rp; V.kof = kof.p; V.pshift = pshift.p; V.w0p = w0p.p; V.g0p = g0p.p; V.c6p = c6p.p;
         V.zeta = zeta.p; V.szr = szr.p; V.c4 = c4.p; V.hmax = hmax.p; V.msd = msd.p;
-        V.cn = cn.p; V.dlog = dlog.p; V.wp = wp.p; V.hdgp = hdgp.p;
+        V.cn = cn.p; V.dxdcn = dxdcn.p; V.dlog = dlog.p; V.wp = wp.p; V.hdgp = hdgp.p;
         V.q = q.p; V.dEdcn = dEdcn.p; V.grad = grad.p; V.E = E.p; V.status = status.p;
         V.brad = alpb_on ? ab.brad.p : nullptr;
         V.bdiag = alpb_on ? ab.bdiag.p : nullptr;
@@ -1660,7 +1660,7 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
         P.x_a.upload(xa); P.x_x.upload(xx); P.x_b.upload(xb); P.x_pre.upload(xpre); P.x_rv.upload(xrv);
     }
     // ---- per-step buffers ----
-    P.cn.alloc(n); P.dlog.alloc(n); 
+    P.cn.alloc(n); P.dxdcn.alloc(n); P.dlog.alloc(n); 
     P.wp.upload(std::vector<double>((size_t)prows * Rp, 0.0));     // zero outside each atom's element
     P.hdgp.upload(std::vector<double>((size_t)prows * Rp, 0.0));   // and in the gaps between molecules
     P.etot.alloc(nm);
@@ -2390,10 +2390,18 @@ void Engine::launch_body()
     P.mark(1);
     const int* cn_off = P.cnl_on ? P.cnl_off.p : nullptr;
     const unsigned watoms = nblk((long)n * 32);
-    if (V.cell.on)
-        (mixed ? k_cn_d4<float, true> : k_cn_d4<double, true>)<<<watoms, kBlock, 0, s>>>(V, nullptr, nullptr, nullptr);
-    else
-        (mixed ? k_cn_d4<float, false> : k_cn_d4<double, false>)<<<watoms, kBlock, 0, s>>>(V, cn_off, P.cnl_j.p, P.cnl_bad.p);
+    auto cn_d4 = [&](auto cell, auto na) {
+        constexpr bool C = decltype(cell)::value;
+        constexpr int NA = decltype(na)::value;
+        const unsigned g = nblk((long)((n + NA - 1) / NA) * 32);
+        const int* off = C ? nullptr : cn_off;
+        if (mixed) k_cn_d4<float, C, NA><<<g, kBlock, 0, s>>>(V, off, P.cnl_j.p, P.cnl_bad.p);
+        else k_cn_d4<double, C, NA><<<g, kBlock, 0, s>>>(V, off, P.cnl_j.p, P.cnl_bad.p);
+    };
+    using One = std::integral_constant<int, 1>;
+    using Four = std::integral_constant<int, 4>;
+    if (V.cell.on) n >= 8192 ? cn_d4(std::true_type{}, Four{}) : cn_d4(std::true_type{}, One{});
+    else n >= 8192 ? cn_d4(std::false_type{}, Four{}) : cn_d4(std::false_type{}, One{});
     P.mark(2);
     if (early) {
         CK(cudaEventRecord(P.ev_fork1, s));

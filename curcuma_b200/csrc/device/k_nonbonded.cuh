@@ -146,21 +146,33 @@ __device__ __forceinline__ void cn_partners(const View& V, int i, const double4&
     }
 }
 
-template <class R, bool CELL>
+// NA: atoms per warp, one after the other for the CN and side by side (eight lanes each) for the
+// weights, whose logarithms and exponentials are the larger part of a large system's time (51,000
+// atoms: 58 us with one atom a warp); one where there are warps to spare.
+template <class R, bool CELL, int NA>
 __global__ void __launch_bounds__(kBlock) k_cn_d4(View V, const int* __restrict__ off, const int* __restrict__ nbr,
                                                  const int* nl_bad)
 {
     constexpr unsigned full = 0xffffffffu;
-    const int i = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (i >= V.n) return;
-    const double4 pi = V.pos[i];
-    const double ri = V.rcov_cn[i];
+    const int lane = threadIdx.x & 31, sub = NA == 1 ? 0 : lane >> 3;
+    const int i0 = (blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5)) * NA;
+    if (i0 >= V.n) return;
     double s = 0.0;
-    cn_partners<CELL>(V, i, pi, off, nbr, nl_bad, [&](int j, double, double, double, double d2) {
-        s += cn_count<R>(d2, ri + V.rcov_cn[j]);
-    });
+#pragma unroll 1
+    for (int a = 0; a < NA; ++a) {
+        const int ia = min(i0 + a, V.n - 1);
+        const double4 pi = V.pos[ia];
+        const double ri = V.rcov_cn[ia];
+        double t = 0.0;
+        cn_partners<CELL>(V, ia, pi, off, nbr, nl_bad, [&](int j, double, double, double, double d2) {
+            t += cn_count<R>(d2, ri + V.rcov_cn[j]);
+        });
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(full, s, o);
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(full, t, o);
+        if (sub == a) s = t;
+    }
+    const int i = min(i0 + sub, V.n - 1);
+    const bool act = i0 + sub < V.n;
     const double cnmax = 4.4;
     const double cn = log(1.0 + exp(cnmax)) - log(1.0 + exp(cnmax - s));
     const int nr = V.nref[i], r = lane & 7;
@@ -188,21 +200,23 @@ __global__ void __launch_bounds__(kBlock) k_cn_d4(View V, const int* __restrict_
     }
     const double z = V.zeta[i];
     const int row = i + V.pshift[V.nmol == 1 ? 0 : V.mol[i]];
-    if (lane == 0) {
+    const int l = NA == 1 ? lane : r;   // lane among those of the atom
+    if (act && l == 0) {
         V.cn[i] = cn;
         V.dlog[i] = exp(cnmax) / (exp(cnmax) + exp(s));
+        V.dxdcn[i] = V.cnf[i] / (2.0 * sqrt(fmax(cn, 0.0)) + 1e-16);
     }
-    if (lane < nr) V.wp[pk(V.Rp, row, V.kof[i] + lane)] = z * w;
+    if (act && l < nr) V.wp[pk(V.Rp, row, V.kof[i] + l)] = z * w;
     const double* C = V.c6p + (size_t)V.slot[i] * 7 * V.Rp;
     double dwa[7];
 #pragma unroll
-    for (int a = 0; a < 7; ++a) dwa[a] = __shfl_sync(full, dw, a);
-    for (int k = lane; k < V.Rp; k += 32) {
+    for (int a = 0; a < 7; ++a) dwa[a] = __shfl_sync(full, dw, (lane & 24) + a);
+    for (int k = l; k < V.Rp; k += NA == 1 ? 32 : 8) {
         double dg = 0.0;
 #pragma unroll
         for (int a = 0; a < 7; ++a)
             if (a < nr) dg += dwa[a] * C[a * V.Rp + k];
-        V.hdgp[pk(V.Rp, row, k)] = z * dg;
+        if (act) V.hdgp[pk(V.Rp, row, k)] = z * dg;
     }
 }
 
@@ -458,10 +472,10 @@ struct TailArgs {
 
 __device__ __forceinline__ double chain_weight(const View& V, int i)
 {
-    const double q = V.q[i], cn = fmax(V.cn[i], 0.0);
+    const double q = V.q[i];
     // the EEQ charge response u adds u dx/dCN (exact-gradient mode)
     const double qe = V.u ? q - V.u[i] : q;
-    return V.dlog[i] * (V.dEdcn[i] - qe * V.cnf[i] / (2.0 * sqrt(cn) + 1e-16));
+    return V.dlog[i] * (V.dEdcn[i] - qe * V.dxdcn[i]);
 }
 
 template <bool CELL>
