@@ -2419,17 +2419,26 @@ void Engine::launch_body()
         const bool full = sv == -1 || (sv == Impl::SOLVE_PCG && !P.pcg_lower);
         const bool aug = sv == Impl::SOLVE_TILED;
         if (P.nred > 0) {
-            const long long nt = (P.nred + kMT - 1) / kMT;
-            const unsigned nb = (unsigned)(nt * (nt + 1) / 2);
+            // 128 columns a block once the lower triangle alone gives every SM a few such blocks
+            // (only the lower-triangle solvers reach that size: full stores take the 32-column form)
+            const bool wide = !full && P.nred >= 2048;
+            const dim3 g((P.nred + (wide ? 127 : 31)) / (wide ? 128 : 32), (P.nred + kMT - 1) / kMT);
+            const bool f32 = sv == Impl::SOLVE_PCG && P.pcg_f32;
+            float* m32 = sv == Impl::SOLVE_PCG && P.pcg_ir ? P.Mf.p : nullptr;
+            auto build = [&](auto born, auto cols) {
+                constexpr bool B = decltype(born)::value;
+                constexpr int C = decltype(cols)::value;
+                if (f32) k_eeq_M_tiles<float, B, C><<<g, 256, 0, s>>>(V, P.red2atom.p, P.anchor.p, P.Mf.p, P.lda, 0, nullptr);
+                else k_eeq_M_tiles<double, B, C><<<g, 256, 0, s>>>(V, P.red2atom.p, P.anchor.p, P.M.p, P.lda, full ? 1 : 0, m32);
+            };
+            using C32 = std::integral_constant<int, 32>;
+            using C128 = std::integral_constant<int, 128>;
             if (sv == Impl::SOLVE_PCG && P.pcg_res)
                 ;   // the resident PCG builds its tiles itself
-            else if (sv == Impl::SOLVE_PCG && P.pcg_f32)
-                (P.alpb_on ? k_eeq_M_tiles<float, true> : k_eeq_M_tiles<float, false>)<<<nb, 256, 0, s>>>(
-                    V, P.red2atom.p, P.anchor.p, P.Mf.p, P.lda, 0, nullptr);
+            else if (P.alpb_on)
+                wide ? build(std::true_type{}, C128{}) : build(std::true_type{}, C32{});
             else
-                (P.alpb_on ? k_eeq_M_tiles<double, true> : k_eeq_M_tiles<double, false>)<<<nb, 256, 0, s>>>(
-                    V, P.red2atom.p, P.anchor.p, P.M.p, P.lda, full ? 1 : 0,
-                    sv == Impl::SOLVE_PCG && P.pcg_ir ? P.Mf.p : nullptr);
+                wide ? build(std::false_type{}, C128{}) : build(std::false_type{}, C32{});
         }
         P.mark(4);
         if (P.nred > 0)

@@ -38,98 +38,92 @@ __device__ __forceinline__ double eeq_a(const View& V, int a, int b)
     return erf(r / sqrt(s)) / r + born;
 }
 
-// reduced matrix, column-major with leading dimension lda: M[c*lda + r]; lower triangle
-// only unless full.  Each thread keeps its row's atoms in registers and walks the
-// columns blockIdx.y, blockIdx.y + gridDim.y, ...
-__global__ void k_eeq_M(View V, const int* __restrict__ red2atom, const int* __restrict__ anchor, double* M,
-                        int lda, int full)
-{
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= V.nred) return;
-    const int k = red2atom[r], ak = anchor[k];
-    for (int c = blockIdx.y; c < V.nred; c += gridDim.y) {
-        if (!full && r < c) continue;
-        const int l = red2atom[c], al = anchor[l];
-        M[(size_t)c * lda + r] = eeq_a(V, k, l) - eeq_a(V, k, al) - eeq_a(V, ak, l) + eeq_a(V, ak, al);
-    }
-}
-
-// Reduced matrix by 32 x 32 tiles of the lower triangle (block (tr, tc), tr >= tc): the
-// tile's row and column atoms (and their anchors) are staged in shared memory, every
-// entry is computed once and written to (r, c) and, when full, to (c, r) through a
-// shared-memory transpose so that both writes are coalesced.
+// Reduced matrix by strips of 32 rows x COLS columns (a grid over strips and rows; strips above the
+// diagonal leave at once): the strip's row and column atoms and their anchors are staged in shared
+// memory, a warp takes COLS / 8 consecutive columns, its lanes the rows, and columns of one
+// fragment share the two elements with their anchor (2 + 2 / (columns of the fragment) elements an
+// entry instead of 4).  With full, the transposed entries go through shared memory, 32 columns at
+// a time, so that both writes are coalesced.  COLS: a block's start is three dependent loads
+// (unknown, anchor, position), ~2 us, which 32 columns do not pay for on large systems: 14,440
+// unknowns (FP64 and FP32 copies, 1.25 GB) 0.87 ms by 32 x 32 tiles with four elements an entry.
 constexpr int kMT = 32;
 // BORN: the ALPB Born matrix enters (V.brad, V.bdiag); the gas-phase instantiation has none of
 // its code
-template <class TM, bool BORN = false>   // storage type of M: double, or float for the FP32-stored PCG matrix
+template <class TM, bool BORN, int COLS>   // storage type of M: double, or float for the FP32-stored PCG matrix
 __global__ void __launch_bounds__(256) k_eeq_M_tiles(View V, const int* __restrict__ red2atom,
                                                     const int* __restrict__ anchor, TM* M, int lda, int full,
-                                                    float* M32 = nullptr)   // optional FP32 copy (k_pcg_ir)
+                                                    float* M32)   // optional FP32 copy (k_pcg_ir)
 {
-    __shared__ double px[4][kMT], py[4][kMT], pz[4][kMT], pa[4][kMT];   // rows k, rows ak, cols l, cols al
-    __shared__ double pbr[4][BORN ? kMT : 1];                            // Born radii (solvation)
-    __shared__ int pid[4][kMT];
+    // row atoms k, their anchors, column atoms l, their anchors: {x, y, z, alpha, Born radius}
+    __shared__ double prow[2][5][kMT], pcol[2][5][COLS];
+    __shared__ int irow[2][kMT], icol[2][COLS];
     __shared__ double T[kMT][kMT + 1];
-    // triangular block index -> (tr, tc)
-    const long long b = blockIdx.x;
-    int tr = (int)((sqrt(8.0 * (double)b + 1.0) - 1.0) * 0.5);
-    while ((long long)(tr + 1) * (tr + 2) / 2 <= b) ++tr;
-    while ((long long)tr * (tr + 1) / 2 > b) --tr;
-    const int tc = (int)(b - (long long)tr * (tr + 1) / 2);
-    const int r0 = tr * kMT, c0 = tc * kMT, n = V.nred;
-    if (threadIdx.x < 4 * kMT) {
-        const int w = threadIdx.x / kMT, t = threadIdx.x % kMT;
-        const int idx = (w < 2 ? r0 : c0) + t;
-        int a = -1;
-        if (idx < n) {
-            const int k = red2atom[idx];
-            a = (w & 1) ? anchor[k] : k;
-        }
-        pid[w][t] = a;
-        if (a >= 0) {
-            const double4 p = V.pos[a];
-            px[w][t] = p.x; py[w][t] = p.y; pz[w][t] = p.z; pa[w][t] = V.alpeeq[a];
-            if constexpr (BORN) pbr[w][t] = V.brad[a];
-        }
+    const int r0 = blockIdx.y * kMT, c0 = blockIdx.x * COLS, n = V.nred;
+    if (c0 > r0 + kMT - 1) return;
+    for (int t = threadIdx.x; t < 2 * (kMT + COLS); t += 256) {
+        const bool row = t < 2 * kMT;
+        const int u = row ? t : t - 2 * kMT, len = row ? kMT : COLS, w = u / len, i = u % len;
+        const int idx = min((row ? r0 : c0) + i, n - 1);   // entries past the end are not written
+        int a = red2atom[idx];
+        if (w) a = anchor[a];
+        const double4 p = V.pos[a];
+        double* d = row ? &prow[w][0][i] : &pcol[w][0][i];
+        d[0] = p.x; d[len] = p.y; d[2 * len] = p.z; d[3 * len] = V.alpeeq[a];
+        if (BORN) d[4 * len] = V.brad[a];
+        (row ? irow[w] : icol[w])[i] = a;
     }
     __syncthreads();
-    auto el = [&](int wa, int ia, int wb, int ib) {
-        if (pid[wa][ia] == pid[wb][ib]) {
-            if constexpr (BORN) return V.adiag[pid[wa][ia]] + V.bdiag[pid[wa][ia]];
-            else return V.adiag[pid[wa][ia]];
-        }
-        const double dx = px[wa][ia] - px[wb][ib], dy = py[wa][ia] - py[wb][ib], dz = pz[wa][ia] - pz[wb][ib];
-        const double d2 = dx * dx + dy * dy + dz * dz;
-        const double s = pa[wa][ia] + pa[wb][ib];
-        if constexpr (!BORN) {
-            if (d2 >= 36.0 * s) return rsqrt(d2);
-            const double r = sqrt(d2);
-            return erf(r / sqrt(s)) / r;
-        } else {
-            const double born = born_p16(V.keps, sqrt(d2), pbr[wa][ia], pbr[wb][ib]);
-            if (d2 >= 36.0 * s) return rsqrt(d2) + born;
-            const double r = sqrt(d2);
-            return erf(r / sqrt(s)) / r + born;
-        }
+    struct RowAtom {
+        double x, y, z, h, al, br;
+        int id;
     };
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;   // 32 x 8
-    for (int cc = ty; cc < kMT; cc += 8) {
-        const int r = r0 + tx, c = c0 + cc;
-        double v = 0.0;
-        if (r < n && c < n) v = el(0, tx, 2, cc) - el(0, tx, 3, cc) - el(1, tx, 2, cc) + el(1, tx, 3, cc);
-        T[cc][tx] = v;
-        if (r < n && c < n && (full || r >= c)) {
-            M[(size_t)c * lda + r] = (TM)v;
-            if (M32) M32[(size_t)c * lda + r] = (float)v;
+    auto row_atom = [&](int w) {
+        return RowAtom{prow[w][0][tx], prow[w][1][tx], prow[w][2][tx], 36.0 * prow[w][3][tx], prow[w][3][tx],
+                       BORN ? prow[w][4][tx] : 0.0, irow[w][tx]};
+    };
+    // A of the row atom with column atom (w, c)
+    auto el = [&](const RowAtom& A, int w, int c) {
+        const double dx = A.x - pcol[w][0][c], dy = A.y - pcol[w][1][c], dz = A.z - pcol[w][2][c];
+        const double d2 = dx * dx + dy * dy + dz * dz, al = pcol[w][3][c];
+        const double ir = rsqrt_pos(d2);
+        double v = ir;
+        if (d2 <= fma(36.0, al, A.h)) {   // inside the charges' width, or the atom itself
+            const double r = d2 * ir;
+            v = A.id == icol[w][c] ? V.adiag[A.id] : erf(r * rsqrt_pos(A.al + al)) * ir;
+        }
+        if (BORN) v += A.id == icol[w][c] ? V.bdiag[A.id] : born_p16(V.keps, d2 * ir, A.br, pcol[w][4][c]);
+        return v;
+    };
+    const RowAtom k = row_atom(0), ak = row_atom(1);
+    const int r = r0 + tx;
+    constexpr int PER = COLS < 4 * 32 ? 4 : COLS / 8;   // consecutive columns of a warp
+    double ka = 0.0, aa = 0.0;
+    int prev = -1;
+    for (int cb = 0; cb < COLS; cb += 8 * PER) {
+        for (int q = 0; q < PER; ++q) {
+            const int cc = cb + PER * ty + q, c = c0 + cc;
+            if (c >= n || c > r0 + kMT - 1) break;   // uniform in the warp
+            if (icol[1][cc] != prev) {
+                prev = icol[1][cc];
+                ka = el(k, 1, cc);
+                aa = el(ak, 1, cc);
+            }
+            const double v = el(k, 0, cc) - ka - el(ak, 0, cc) + aa;
+            if (r < n && (full || r >= c)) {
+                M[(size_t)c * lda + r] = (TM)v;
+                if (M32) M32[(size_t)c * lda + r] = (float)v;
+            }
+            if (full && COLS == kMT) T[cc][tx] = v;
         }
     }
-    if (!full || tr == tc) return;
+    if (!full || COLS != kMT || r0 == c0) return;
     __syncthreads();
     for (int rr = ty; rr < kMT; rr += 8) {   // (c, r) entries: row c0 + tx of column r0 + rr
-        const int r = r0 + rr, c = c0 + tx;
-        if (r < n && c < n) {
-            M[(size_t)r * lda + c] = (TM)T[tx][rr];
-            if (M32) M32[(size_t)r * lda + c] = (float)T[tx][rr];
+        const int r2 = r0 + rr, c = c0 + tx;
+        if (r2 < n && c < n) {
+            M[(size_t)r2 * lda + c] = (TM)T[tx][rr];
+            if (M32) M32[(size_t)r2 * lda + c] = (float)T[tx][rr];
         }
     }
 }
