@@ -745,6 +745,7 @@ struct Engine::Impl {
     DBuf<double> px, pz, ppartial;
     DBuf<unsigned int> pbar;
     DBuf<int> piters;
+    bool pcg_big = false;   // preconditioner blocks of more than kPcgRowThread rows
     int pcg_grid = 0, pcg_max_iter = 200, pcg_maxrows = 1, pcg_maxinv = 1;
     size_t pcg_smem = 0;
     bool pcg_ready = false;
@@ -813,6 +814,7 @@ struct Engine::Impl {
             A.inner_rel = er ? std::atof(er) : 1e-6;
         }
         A.binv_pre = pcg_pre ? pbinv.p : nullptr;
+        A.big = pcg_big;
         void* args[] = {&A};
         if (pcg_ir) {
             void* irargs[] = {&A, &pcg_tmap};
@@ -1736,7 +1738,7 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
             const char* ep = std::getenv("GFNFF_PCG_PRE");
             P.pcg_pre = big > kPcgWarpMax && !(ep && !std::strcmp(ep, "0"));
             if (P.pcg_pre) {
-                blkmax = 128;
+                blkmax = 512;   // whole fragments: 353 atoms in 1500 waters take 13 iterations, 47 in blocks of 128
                 if (const char* eb = std::getenv("GFNFF_PCG_PREBLK")) blkmax = std::max(2, std::min(512, std::atoi(eb)));
             }
         }
@@ -1829,14 +1831,19 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
             std::vector<int4> part;
             std::vector<long long> boff;
             long long bo = 0;
-            for (auto& b : blocks) { boff.push_back(bo); bo += (long long)b.y * b.y; }
+            P.pcg_big = false;
+            for (auto& b : blocks) {
+                boff.push_back(bo);
+                bo += (long long)b.y * b.y;
+                P.pcg_big = P.pcg_big || b.y > kPcgRowThread;
+            }
             // the lower-triangle form from 4096 unknowns (the matrix leaves L2), and for chains
-            // with set-up block inverses from 1024: its tiled product balances work by tiles, so
+            // with set-up block inverses from 256: its tiled product balances work by tiles, so
             // every SM takes part even where large preconditioner blocks, owned whole, would
             // load a few blocks with most rows (Gly50 + 1500 waters: 1.45 -> 0.69 ms)
             const char* esym = std::getenv("GFNFF_PCG_SYM");
             const bool lower = esym ? std::strcmp(esym, "0") != 0
-                                    : (P.nred >= 4096 || (P.pcg_pre && P.nred >= 1024));
+                                    : (P.nred >= 4096 || (P.pcg_pre && P.nred >= 256));
             const int G = lower ? nsm : std::max(1, std::min(nsm, (int)blocks.size()));
             size_t bk = 0;
             int maxrows = 1;

@@ -45,6 +45,7 @@ struct PCGArgs {
     int* warm;            // when non-null and *warm != 0, x holds the previous solution of the
                           // same system and is the initial guess; set to 1 on convergence
     const float* Mf;      // lower form in the mixed precision form: M stored in FP32 (M unused)
+    bool big;             // there are preconditioner blocks of more than kPcgRowThread rows
     const double* binv_pre;   // block inverses computed at set-up (global memory, boff layout), or null
     int lower;            // 1 or 2: only the lower triangle of M is stored; M p by tiles
                           // (matvec_tiles, streaming 4 or 8 columns per warp at once)
@@ -177,21 +178,63 @@ __device__ void update_p(double* p, const double* z, int n, double beta)
     }
 }
 
-// z = P^-1 r on the owned rows (one thread per row, rblk[r] = its preconditioner block),
-// everything in shared memory: r, z and the block inverses of this grid block; returns
-// the thread's part of r.z
-// meta[k] = {first local row of row k's block, block size, offset of row k's inverse row}
-__device__ double apply_precond(int nrow, const int4* meta, const double* binv, const double* r, double* z)
+// z = P^-1 r on the owned rows (rblk[r] = the row's preconditioner block); r and z in shared
+// memory, the block inverses there or (computed at set-up) in global memory; returns the thread's
+// part of r.z.  meta[k] = {first local row of row k's block, block size, offset of row k's inverse
+// row}.  Rows of blocks up to kPcgRowThread one per thread; rows of larger blocks (big: there are
+// any) four at a time by a warp, lanes along the row: with a thread per row no two lanes shared a
+// line of the inverse, and the product took most of an iteration of a solvated chain.
+constexpr int kPcgRowThread = 8;
+__device__ __noinline__ double apply_precond_big(int nrow, const int4* meta, const double* binv, const double* r,
+                                                 double* z)
+{
+    double rz = 0.0;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    for (int k0 = 4 * warp; k0 < nrow; k0 += 4 * nw) {
+        int4 m[4];
+        double s[4] = {0.0, 0.0, 0.0, 0.0};
+        int most = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            m[i] = meta[min(k0 + i, nrow - 1)];
+            most = max(most, m[i].y);
+        }
+        if (most <= kPcgRowThread) continue;   // uniform in the warp
+#pragma unroll 2
+        for (int j = lane; j < most; j += 32)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (j < m[i].y) s[i] += binv[m[i].z + j] * r[m[i].x + j];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s[i] += __shfl_xor_sync(0xffffffffu, s[i], o);
+        const double t = lane < 2 ? (lane == 0 ? s[0] : s[1]) : (lane == 2 ? s[2] : s[3]);
+        const int y = lane < 2 ? (lane == 0 ? m[0].y : m[1].y) : (lane == 2 ? m[2].y : m[3].y);
+        if (lane < 4 && k0 + lane < nrow && y > kPcgRowThread) {
+            z[k0 + lane] = t;
+            rz += t * r[k0 + lane];
+        }
+    }
+    return rz;
+}
+
+__device__ double apply_precond(int nrow, const int4* meta, const double* binv, const double* r, double* z, bool big)
 {
     double rz = 0.0;
     for (int k = threadIdx.x; k < nrow; k += blockDim.x) {
         const int4 m = meta[k];
+        if (m.y > kPcgRowThread) continue;
         const double* Bi = binv + m.z;
         const double* rb = r + m.x;
         double s = 0.0;
         for (int j = 0; j < m.y; ++j) s += Bi[j] * rb[j];
         z[k] = s;
         rz += s * r[k];
+    }
+    if (big) {
+        rz += apply_precond_big(nrow, meta, binv, r, z);
+        __syncthreads();   // the callers read z with a thread per row
     }
     return rz;
 }
@@ -533,7 +576,7 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcg(PCGArgs A)
         bmax_t = fmax(bmax_t, fabs(bv));
     }
     __syncthreads();
-    double rz_t = apply_precond(nrow, meta, Bp, rs, zs);
+    double rz_t = apply_precond(nrow, meta, Bp, rs, zs, A.big);
     for (int k = threadIdx.x; k < nrow; k += blockDim.x) __stcg(A.z + row0 + k, zs[k]);
     // the start totals have a slot of their own: a fast block writes its first p.Mp
     // partial into slot 0 before a slow one has read these after the barrier
@@ -562,7 +605,7 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcg(PCGArgs A)
             rmax_t = fmax(rmax_t, fabs(rs[k]));
         }
         __syncthreads();
-        rz_t = apply_precond(nrow, meta, Bp, rs, zs);
+        rz_t = apply_precond(nrow, meta, Bp, rs, zs, A.big);
         for (int k = threadIdx.x; k < nrow; k += blockDim.x) __stcg(A.z + row0 + k, zs[k]);
         block_sum_max(rz_t, rmax_t, A.partial + 8 * blockIdx.x + 2);
         ok = grid_sync(A.bar, gen);
@@ -591,7 +634,7 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcg(PCGArgs A)
                 rmax_t = fmax(rmax_t, fabs(rs[k]));
             }
             __syncthreads();
-            rz_t = apply_precond(nrow, meta, Bp, rs, zs);
+            rz_t = apply_precond(nrow, meta, Bp, rs, zs, A.big);
             for (int k = threadIdx.x; k < nrow; k += blockDim.x) __stcg(A.z + row0 + k, zs[k]);
             block_sum_max(rz_t, rmax_t, A.partial + 8 * blockIdx.x + 2);
             ok = grid_sync(A.bar, gen);
@@ -880,7 +923,7 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcg_ir(PCGArgs A, const __grid_
             rmax_t = fmax(rmax_t, fabs(r));
         }
         __syncthreads();
-        double rz_t = apply_precond(nrow, meta, Bp, rs, zs);
+        double rz_t = apply_precond(nrow, meta, Bp, rs, zs, A.big);
         for (int k = threadIdx.x; k < nrow; k += blockDim.x) __stcg(A.z + row0 + k, zs[k]);
         block_sum_max(rz_t, rmax_t, A.partial + 8 * blockIdx.x + 4);
         ok = grid_sync(A.bar, gen);
@@ -916,7 +959,7 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcg_ir(PCGArgs A, const __grid_
                 rin_t = fmax(rin_t, fabs(rs[k]));
             }
             __syncthreads();
-            rz_t = apply_precond(nrow, meta, Bp, rs, zs);
+            rz_t = apply_precond(nrow, meta, Bp, rs, zs, A.big);
             for (int k = threadIdx.x; k < nrow; k += blockDim.x) __stcg(A.z + row0 + k, zs[k]);
             block_sum_max(rz_t, rin_t, A.partial + 8 * blockIdx.x + 2);
             ok = grid_sync(A.bar, gen);
@@ -1077,7 +1120,7 @@ __global__ void __launch_bounds__(kPcgPipeThreads, 2) k_pcg_pipe(PCGArgs A)
         bmax_t = fmax(bmax_t, fabs(bv));
     }
     __syncthreads();
-    apply_precond(nrow, meta, Bp, rs, us);
+    apply_precond(nrow, meta, Bp, rs, us, A.big);
     double bmax = 0.0, t1, t2;
     publish(us, 0.0, 0.0, bmax_t, t1, t2, bmax);
     product(ws);
@@ -1092,7 +1135,7 @@ __global__ void __launch_bounds__(kPcgPipeThreads, 2) k_pcg_pipe(PCGArgs A)
             rm_t = fmax(rm_t, fabs(rs[k]));
         }
         __syncthreads();
-        apply_precond(nrow, meta, Bp, ws, ms);
+        apply_precond(nrow, meta, Bp, ws, ms, A.big);
         double gam, del, rmax;
         publish(ms, g_t, d_t, rm_t, gam, del, rmax);
         if (!ok) break;
@@ -1108,7 +1151,7 @@ __global__ void __launch_bounds__(kPcgPipeThreads, 2) k_pcg_pipe(PCGArgs A)
                 rt = fmax(rt, fabs(rs[k]));
             }
             __syncthreads();
-            apply_precond(nrow, meta, Bp, rs, us);
+            apply_precond(nrow, meta, Bp, rs, us, A.big);
             double rtrue;
             publish(us, 0.0, 0.0, rt, u1, u2, rtrue);
             if (!ok) break;
@@ -1340,7 +1383,7 @@ __global__ void __launch_bounds__(kPcgPipeThreads, 1) k_pcg_res(PCGArgs A, PCGRe
         bmax_t = fmax(bmax_t, fabs(bv));
     }
     __syncthreads();
-    apply_precond(nrow, meta, Bp, rs, us);
+    apply_precond(nrow, meta, Bp, rs, us, A.big);
     double bmax = 0.0, t1, t2;
     publish(us, 0.0, 0.0, bmax_t, t1, t2, bmax);
     product(ws);
@@ -1355,7 +1398,7 @@ __global__ void __launch_bounds__(kPcgPipeThreads, 1) k_pcg_res(PCGArgs A, PCGRe
             rm_t = fmax(rm_t, fabs(rs[k]));
         }
         __syncthreads();
-        apply_precond(nrow, meta, Bp, ws, ms);
+        apply_precond(nrow, meta, Bp, ws, ms, A.big);
         double gam, del, rmax;
         publish(ms, g_t, d_t, rm_t, gam, del, rmax);
         if (!ok) break;
@@ -1370,7 +1413,7 @@ __global__ void __launch_bounds__(kPcgPipeThreads, 1) k_pcg_res(PCGArgs A, PCGRe
                 rt = fmax(rt, fabs(rs[k]));
             }
             __syncthreads();
-            apply_precond(nrow, meta, Bp, rs, us);
+            apply_precond(nrow, meta, Bp, rs, us, A.big);
             double rtrue;
             publish(us, 0.0, 0.0, rt, u1, u2, rtrue);
             if (!ok) break;
