@@ -3,17 +3,17 @@
 // Pipeline of one evaluation (single stream, every buffer device-resident):
 //   positions -> CN (erf counting, 6 bohr) -> D4 Gaussian weights + half contraction
 //   -> EEQ: reduced Coulomb matrix built from the geometry, fragment constraints
-//      eliminated in the null space, Cholesky solve -> charges
+//      eliminated in the null space, iterative or direct solve -> charges
 //   -> bonded terms (bond/angle/torsion/inversion/sTors/BATM/ATM/HB/XB, one thread per
 //      term, gradient scattered with FP64 atomics)
-//   -> repulsion (per-atom CSR lists) and all-pairs Coulomb + D4 dispersion (shared-
-//      memory partner tiles)
-//   -> self energy, CN chain rule (dE/dCN - q*cnf/(2 sqrt CN)) * dCN/dr, outputs.
+//   -> repulsion (per-atom CSR lists) and all-pairs Coulomb and D4 dispersion (register
+//      tiles of pairs)
+//   -> CN chain rule (dE/dCN - q*cnf/(2 sqrt CN)) * dCN/dr, outputs.
 //
 // The engine holds one molecule or a batch of independent molecules: atoms are stored
 // molecule by molecule, Morton-sorted inside each molecule, and every pair loop is
 // restricted to the atom's own molecule.  The EEQ of a batch is block diagonal and is
-// solved by one thread block per molecule.
+// solved by one thread block or cluster per molecule.
 //
 // Every kernel restates the curcuma routine cited beside it (paths relative to
 // src/core/energy_calculators/ff_methods/).
