@@ -8,7 +8,7 @@ charges of these matrices (smallest eigenvalue >= 0.1) then agree to 1e-11 at wo
 import numpy as np
 import pytest
 
-from curcuma_b200 import FP64, GFNFF, workloads
+from curcuma_b200 import FP64, GFNFF, MIXED, workloads
 from tests.indefinite_systems import h2_chain
 from tests.oracle_api import Oracle
 
@@ -65,3 +65,36 @@ def test_batch_with_indefinite_molecule(monkeypatch):
     assert (s0 == s1).all()
     assert s0[0] == 0 and s0[2] == 0
     assert np.abs(e0 - e1).max() < 1e-9
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("setup_bond", [0.471, 0.74])
+def test_indefinite_with_a_symmetric_right_hand_side(setup_bond, precision, monkeypatch):
+    """H2 at 0.471 A: one unknown, a negative matrix and a right-hand side of zero; four of them on
+    the corners of a square (tilted, so that the matrix has no zeros) have right-hand sides without
+    the antisymmetric modes.  Both are not positive definite whatever the right-hand side, as the
+    Cholesky kernel says, and whichever molecules they are evaluated with."""
+    z = np.array([1, 1], dtype=np.int32)
+
+    def square(bond):
+        u = bond / 2 * np.array([0.6, 0.8, 0.0])
+        v = bond / 2 * np.array([-0.8, 0.6, 0.0])
+        c = 4.0 * np.array([[1, 0, 0], [0, 1, 0], [-1, 0, 0], [0, -1, 0]])
+        return np.concatenate([np.stack([c[k] - (v if k % 2 else u), c[k] + (v if k % 2 else u)]) for k in range(4)])
+
+    def mols(bond):
+        return [workloads.alkane(8, 1), (z, np.array([[0.0, 0, 0], [bond, 0, 0]])),
+                (np.tile(z, 4), square(bond)), workloads.alkane(50, 2)]
+
+    for direct in (False, True):
+        if direct:
+            monkeypatch.setenv("GFNFF_BATCH_TC", "0")
+        g = GFNFF(precision=precision)
+        assert g.setMoleculeBatch(mols(setup_bond)), g.getErrorMessage()
+        g.updateGeometry(np.concatenate([x for _, x in mols(0.471)]))
+        e, st = g.calculateEnergyBatch()
+        assert list(st) == [0, 3, 3, 0], (direct, st)   # 3: GFNFF_NOT_SPD
+        g.updateGeometry(np.concatenate([x for _, x in mols(0.74)]))   # and definite here
+        e, st = g.calculateEnergyBatch()
+        assert (st == 0).all(), (direct, st)
+        assert np.abs(g.getCharges()[26:28]).max() == 0.0
