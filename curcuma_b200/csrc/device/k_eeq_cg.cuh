@@ -173,19 +173,23 @@ __device__ __forceinline__ void cg_product(const T* A, int ld, int rows, int row
     }
 }
 
-// r.z, z.w and max |r| (rounded up to FP32), the same in every warp
+// |v| rounded up to FP32, as bits, which order as the values with NaN above all: a maximum over them
+// keeps a NaN (fmaxf drops it), so that no bound on it holds
+__device__ __forceinline__ unsigned abs_bits(double v) { return __float_as_uint(__double2float_ru(fabs(v))); }
+
+// r.z, z.w and max |r|, the same in every warp
 __device__ __forceinline__ void cg_dots(const double* r, const double* z, const double* w, int n, double& rz,
                                         double& zw, float& rmax)
 {
     constexpr unsigned full = 0xffffffffu;
     double a = 0.0, b = 0.0;
-    float m = 0.f;
+    unsigned m = 0;
 #pragma unroll 2
     for (int c = threadIdx.x & 31; c < n; c += 32) {
         const double rc = r[c], zc = z[c];
         a = fma(rc, zc, a);
         b = fma(zc, w[c], b);
-        m = fmaxf(m, __double2float_ru(fabs(rc)));
+        m = max(m, abs_bits(rc));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -194,15 +198,15 @@ __device__ __forceinline__ void cg_dots(const double* r, const double* z, const 
     }
     rz = a;
     zw = b;
-    rmax = __uint_as_float(__reduce_max_sync(full, __float_as_uint(m)));   // non-negative: ordered as the bits
+    rmax = __uint_as_float(__reduce_max_sync(full, m));
 }
 
 // max |v|, the same in every warp
 __device__ __forceinline__ float cg_max(const double* v, int n)
 {
-    float m = 0.f;
-    for (int c = threadIdx.x & 31; c < n; c += 32) m = fmaxf(m, __double2float_ru(fabs(v[c])));
-    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+    unsigned m = 0;
+    for (int c = threadIdx.x & 31; c < n; c += 32) m = max(m, abs_bits(v[c]));
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, m));
 }
 
 // entry c of the start vector, in [-1, 1): the bits of c mixed by multiplications and shifts

@@ -8,7 +8,7 @@ charges of these matrices (smallest eigenvalue >= 0.1) then agree to 1e-11 at wo
 import numpy as np
 import pytest
 
-from curcuma_b200 import FP64, GFNFF, MIXED, workloads
+from curcuma_b200 import FP64, GFNFF, MIXED, _lib, workloads
 from tests.indefinite_systems import h2_chain
 from tests.oracle_api import Oracle
 
@@ -98,3 +98,30 @@ def test_indefinite_with_a_symmetric_right_hand_side(setup_bond, precision, monk
         e, st = g.calculateEnergyBatch()
         assert (st == 0).all(), (direct, st)
         assert np.abs(g.getCharges()[26:28]).max() == 0.0
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED], ids=["fp64", "mixed"])
+def test_coordinate_that_is_not_a_number(precision, monkeypatch):
+    """Through the device entry point, which cannot look at its coordinates: the molecule's matrix holds
+    NaN, and it gets the status that the Cholesky kernel gives it; its neighbours are not touched."""
+    import torch
+
+    mols = [workloads.alkane(8, 1), workloads.alkane(20, 3), workloads.alkane(50, 2)]
+    x = np.concatenate([x for _, x in mols]) / 0.529177210903
+    x[30, 1] = np.nan
+    d_x = torch.from_numpy(x).cuda()
+    for direct in (False, True):
+        if direct:
+            monkeypatch.setenv("GFNFF_BATCH_TC", "0")
+        g = GFNFF(precision=precision)
+        assert g.setMoleculeBatch(mols), g.getErrorMessage()
+        e, _ = g.calculateEnergyBatch()
+        d_e = torch.zeros(3, dtype=torch.float64, device="cuda")
+        d_st = torch.full((3,), -1, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        st = _lib.load().gfnff_energy_and_gradient_device(g.handle, d_x.data_ptr(), d_e.data_ptr(), None,
+                                                          d_st.data_ptr())
+        assert st == 0
+        torch.cuda.synchronize()
+        assert d_st.tolist() == [0, 3, 0], (direct, d_st.tolist())
+        assert abs(float(d_e[0]) - e[0]) < 1e-9 and abs(float(d_e[2]) - e[2]) < 1e-9
