@@ -530,9 +530,8 @@ struct Engine::Impl {
     }
     CgArgs cg_args() const
     {
-        // a batch leaves unsolved molecules to k_eeq_batch (-1), a single molecule to the host
         return CgArgs{cg_mols.p, roff.p, red2atom.p, anchor.p, qlist.p, nq, q0.p, cg_pinv.p, cg_poff.p, bvec.p, info.p,
-                      nmol > 1 ? -1 : 1, nmol > 1 ? -1 : 3, cg_iters.p, 500, opt.precision == 1 ? kRefineTol : 0.0};
+                      cg_iters.p, opt.precision == 1 ? kRefineTol : 0.0};
     }
     // one cluster of b.cs CTAs per molecule of the bin
     template <class... P, class... Q>
@@ -2157,7 +2156,7 @@ bool Engine::switch_to_lu()
 bool Engine::switch_to_direct()
 {
     if (p_->nmol != 1) return false;
-    if (p_->solver != Impl::SOLVE_PCG && !(p_->solver == Impl::SOLVE_BATCH && (p_->batch_tc || p_->cg_on))) return false;
+    if (p_->solver != Impl::SOLVE_PCG && !(p_->solver == Impl::SOLVE_BATCH && p_->batch_tc)) return false;
     p_->drop_graphs();
     p_->solver = Impl::SOLVE_TILED;   // the in-house FP64 Cholesky
     return true;
@@ -2474,11 +2473,12 @@ void Engine::launch_body()
         P.mark(4);
         P.mark(5);
         if (fork && !early) CK(cudaEventRecord(P.ev_fork1, s));   // single molecule, batched solver
-        if (P.cg_on) P.cg_launch(V, s);
-        if (!P.cg_on || P.nmol > 1) {   // Cholesky: of every molecule, or of those left over
+        if (P.cg_on) {
+            P.cg_launch(V, s);
+        } else {
             EEQBatch B{P.roff.p, P.moff.p, P.border.p, P.bitems.p, P.nbitems, P.bnext.p, P.batch_smem_max, P.red2atom.p,
                        P.anchor.p, P.qlist.p, P.nq, P.q0.p, P.M.p, P.bvec.p, P.info.p,
-                       P.batch_tc ? 1 : 0, P.M64.p, P.m64off.p, kRefineTol, P.refine.p, P.cg_on ? 1 : 0};
+                       P.batch_tc ? 1 : 0, P.M64.p, P.m64off.p, kRefineTol, P.refine.p};
             if (P.batch_tc && P.n_tc_tiles) k_eeq_tc_tiles<<<P.n_tc_tiles, 256, 0, s>>>(V, B, P.tc_tiles.p);
             k_eeq_batch<<<P.batch_grid, 512, P.batch_smem, s>>>(V, B);
         }

@@ -236,7 +236,6 @@ struct EEQBatch {
     const long long* m64off;
     double tol;             // refinement target ||b - M y||_inf
     int* refine;            // largest number of refinement corrections of the launch
-    int todo;               // only the molecules k_eeq_cg left over (info -1)
 };
 
 __device__ void tc_solve(const View& V, const EEQBatch& P, int m, double* S);
@@ -671,11 +670,10 @@ __global__ void __launch_bounds__(512) k_eeq_batch(View V, EEQBatch P)
         if (it.x < 0) return;
         if (it.z) {   // warp mode: warp w solves molecule order[first + w]
             const int w = threadIdx.x >> 5;
-            if (w < it.y && (!P.todo || P.info[P.order[it.x + w]] == -1)) warp_solve(V, P, P.order[it.x + w], S + (size_t)w * kWarpRegion);
+            if (w < it.y) warp_solve(V, P, P.order[it.x + w], S + (size_t)w * kWarpRegion);
             continue;
         }
         const int m = P.order[it.x];
-        if (P.todo && P.info[m] != -1) continue;
         const int r0 = P.roff[m], nr = P.roff[m + 1] - r0;
         double* y = P.y + r0;
         if (nr == 0) {

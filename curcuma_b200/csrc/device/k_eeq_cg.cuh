@@ -13,8 +13,10 @@
 // Accuracy: the recurrence runs to a residual of 1e-15 max|b| (FP64 form; the rounding level of a
 // direct solve) or half the absolute bar (mixed form), and the result is accepted on the true FP64
 // residual b - M x: at most 1e-12 max|b|, or the bar.  A search direction with p M p <= 0 (M not
-// positive definite) or too many iterations leaves the molecule to the Cholesky kernel
-// (k_eeq_batch), which decides its status.
+// positive definite) or too many iterations (M nearly singular, or far from the set-up geometry)
+// leaves the molecule to a direct elimination in the same kernel (cg_direct), which always ends
+// with a solution or a pivot that is not positive: every entry (single evaluations, device loops,
+// MD, batches) gets the status that a factorisation gives.
 //
 // Definiteness: CG meets a negative direction only if its residual has a part along it (then it
 // cannot converge past it: with positive Ritz values only, the residual polynomial grows on the
@@ -37,10 +39,8 @@ struct CgArgs {
     const float* pinv;      // inverses at the set-up geometry, rows of cg_ld(nr) floats
     const long long* poff;
     double* y;
-    int* info;              // 0; `fail1` (not positive definite), `fail3` (not converged)
-    int fail1, fail3;
+    int* info;              // 0, or 1: not positive definite
     int* iters;             // largest number of products of the launch
-    int max_iter;
     double tol_abs;         // > 0: the mixed form's bar
 };
 
@@ -219,6 +219,54 @@ __device__ __forceinline__ double cg_start(int c)
     return (double)(int)h * 0x1p-31;
 }
 
+// Gauss-Jordan elimination of M x = b on the cluster's row slices, without pivoting (M symmetric: a
+// pivot that is not positive means that it is not positive definite).  The owner of row k stores it
+// into every CTA, two buffers in turn: the one of step k + 2 is written after the barrier of step
+// k + 1, which every CTA reaches with its reads of step k done.  M and the slice of b are used up;
+// x goes to y.  True if every pivot was positive, the same in every CTA.  A barrier a row: 38 us for
+// 25 unknowns, 140 for 91, 350 for 193, 650 for 301 (CG at 0.03 Angstrom noise 30, 51, 69, 79).
+template <int CS>
+__device__ __noinline__ bool cg_direct(double* M, int rows, int row0, int nr, double* b, double* rowbuf, double* bk2,
+                                       double* y)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    cluster_barrier<CS>();   // every CTA is done with its vectors
+    for (int k = 0; k < nr; ++k) {
+        double* row = rowbuf + (k & 1) * nr;
+        double* bk = bk2 + (k & 1);
+        if (k >= row0 && k < row0 + rows) {   // the owner
+            const double* Mk = M + (size_t)(k - row0) * nr;
+            for (int c = threadIdx.x; c < (nr - k) * CS; c += blockDim.x) {
+                const int dst = CS == 1 ? 0 : c / (nr - k), j = k + (CS == 1 ? c : c % (nr - k));
+                if (CS == 1) row[j] = Mk[j];
+                else cluster_store(row + j, dst, Mk[j]);
+            }
+            if (threadIdx.x < CS) {
+                if (CS == 1) *bk = b[k];
+                else cluster_store(bk, threadIdx.x, b[k]);
+            }
+        }
+        cluster_barrier<CS>();
+        const double piv = row[k];
+        if (!(piv > 0.0)) return false;
+        const double inv = 1.0 / piv, bv = *bk;
+        for (int q = warp; q < rows; q += nw) {
+            if (row0 + q == k) continue;
+            double* Mi = M + (size_t)q * nr;
+            const double f = Mi[k] * inv;
+            for (int j = k + 1 + lane; j < nr; j += 32) Mi[j] -= f * row[j];
+            if (lane == 0) b[row0 + q] -= f * bv;
+        }
+        __syncthreads();
+    }
+    for (int q = threadIdx.x; q < rows; q += blockDim.x) y[row0 + q] = b[row0 + q] / M[(size_t)q * nr + row0 + q];
+    return true;
+}
+
+// products after which the elimination is the cheaper end (1.6-5.3 us a product against the times of
+// cg_direct): a solve costs at most about twice the elimination
+__device__ __forceinline__ int cg_max_iter(int nr) { return 20 + 2 * nr / 5; }
+
 constexpr int kCgThreads = 512;   // at most: a warp per four rows of the slice (cg_threads)
 inline int cg_threads(int nr, int cs) { return 64 * std::min(kCgThreads / 64, std::max(2, ((nr + cs - 1) / cs + 7) / 8)); }
 
@@ -311,7 +359,8 @@ __global__ void __launch_bounds__(kCgThreads) k_eeq_cg(View V, CgArgs A)
     const float scale = bmax > 0.f ? bmax : umax;
     const float stop = A.tol_abs > 0.0 ? 0.5f * (float)A.tol_abs : 1e-15f * scale;
     const float accept = A.tol_abs > 0.0 ? (float)A.tol_abs : 1e-12f * scale;
-    int it = 0, state = -1;   // -1: running
+    const int max_iter = cg_max_iter(nr);
+    int it = 0, state = -1;   // -1: running, 0: solved, else left to the elimination
     bool start = true;
     while (state < 0) {
         double* z = z2 + (it & 1) * nr;
@@ -321,7 +370,7 @@ __global__ void __launch_bounds__(kCgThreads) k_eeq_cg(View V, CgArgs A)
         cluster_barrier<CS>();
         ++it;
         cg_dots(r, z, w, nr, rz, zw, rmax);
-        if (!start && (rmax <= stop || it >= A.max_iter)) {   // the true residual decides
+        if (!start && (rmax <= stop || it >= max_iter)) {   // the true residual decides
             cluster_barrier<CS>();   // every CTA has read w
             cg_product<CS, double>(M, nr, rows, row0, nr, x, w);
             cluster_barrier<CS>();
@@ -332,7 +381,7 @@ __global__ void __launch_bounds__(kCgThreads) k_eeq_cg(View V, CgArgs A)
             __syncthreads();
             cg_dots(r, r, r, nr, dummy, zw, rmax);
             if (rmax <= accept) state = 0;
-            else if (it >= A.max_iter) state = 3;
+            else if (it >= max_iter) state = 3;
             start = true;
             continue;
         }
@@ -356,13 +405,16 @@ __global__ void __launch_bounds__(kCgThreads) k_eeq_cg(View V, CgArgs A)
         start = false;
         __syncthreads();
     }
-    if (rank == 0) {
+    if (state != 0) {
+        const bool ok = cg_direct<CS>(M, rows, row0, nr, b, z2, w, A.y + r0);
+        state = ok ? 0 : 1;
+    } else if (rank == 0) {
         __syncthreads();
         for (int q = threadIdx.x; q < nr; q += blockDim.x) A.y[r0 + q] = bmax == 0.f ? 0.0 : x[q];
-        if (threadIdx.x == 0) {
-            A.info[mol] = state == 0 ? 0 : (state == 1 ? A.fail1 : A.fail3);
-            atomicMax(A.iters, it);
-        }
+    }
+    if (rank == 0 && threadIdx.x == 0) {
+        A.info[mol] = state;
+        atomicMax(A.iters, it);
     }
     cluster_barrier<CS>();   // no CTA leaves while another may store into it
 }

@@ -464,7 +464,6 @@ __global__ void __launch_bounds__(256) k_eeq_tc_tiles(View V, EEQBatch P, const 
     __shared__ int s_single;
     const int4 t = tiles[blockIdx.x];
     const int m = t.x, R = t.y, C = t.z;
-    if (P.todo && P.info[m] != -1) return;
     const int r0 = P.roff[m], nr = P.roff[m + 1] - r0;
     const int tid = threadIdx.x;
     if (tid < 128) {

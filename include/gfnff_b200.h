@@ -229,7 +229,7 @@ gfnff_status gfnff_eeq_charges_noalloc(int natoms, int nfrag, const double* d_xy
  * persistent tiled Cholesky), "pcg" (block-Jacobi conjugate gradients; FP64 true residual
  * <= 1e-12 max|b| in the FP64 form, <= 1e-10 in the mixed form), "batched" (per-molecule
  * conjugate gradients with the set-up inverse on a thread-block cluster, to the same FP64
- * residuals; a Cholesky for large batches and where that fails), "lu" (indefinite matrix,
+ * residuals, with a direct elimination where they do not; a Cholesky for large batches), "lu" (indefinite matrix,
  * pivoted LU) or "library" (cuSOLVER's Cholesky, only when GFNFF_EEQ_SOLVER=library asks
  * for it); "" before setup.  The choice is made by timing the in-house solvers at setup.  curcuma's EEQSolver also picks among several solvers
  * (eeq_solver.cpp:1448-2086); this query has no counterpart there. */

@@ -1,6 +1,6 @@
 """The batched EEQ by conjugate gradients with the set-up inverse (k_eeq_cg): sizes at the edges of
 its row groups and on both sides of every cluster size, geometries off the set-up, several
-fragments, and a molecule whose matrix is not positive definite (left to the Cholesky kernel).
+fragments, and molecules whose matrix is not, or hardly, positive definite (left to the elimination).
 
 Tolerances: the FP64 solve is accepted at a true residual of 1e-12 max|b| and runs to 1e-15; the
 charges of these matrices (smallest eigenvalue >= 0.1) then agree to 1e-11 at worst, energies
@@ -125,3 +125,51 @@ def test_coordinate_that_is_not_a_number(precision, monkeypatch):
         torch.cuda.synchronize()
         assert d_st.tolist() == [0, 3, 0], (direct, d_st.tolist())
         assert abs(float(d_e[0]) - e[0]) < 1e-9 and abs(float(d_e[2]) - e[2]) < 1e-9
+
+
+def _near_singular(bond):
+    """H2 between two waters: positive definite from a bond of 0.527 A on"""
+    w = workloads.water_geometry()
+    w = w - w[0]
+    z = np.array([1, 1, 8, 1, 1, 8, 1, 1], dtype=np.int32)
+    h2 = np.array([[0.0, -bond / 2, 0.0], [0.0, bond / 2, 0.0]])
+    return z, np.concatenate([h2, w + np.array([2.9, 0.3, 0.1]), w + np.array([-2.9, 0.7, 1.1])])
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED], ids=["fp64", "mixed"])
+def test_nearly_singular_matrix_on_the_device_entry(precision, monkeypatch):
+    """A matrix that the Cholesky kernel still factorises gets status 0 where nothing on the host can
+    evaluate it again.  One eigenvalue l is almost 0: E ~ -b^2 / (2 l), so an error of some 1e-15 in M
+    (its elements are of order 1) shows as 1e-15 / l = 1e-15 * 2 |E| / b^2 of E; b^2 > 1e-5 here."""
+    import torch
+
+    lib = _lib.load()
+    d_e = torch.zeros(1, dtype=torch.float64, device="cuda")
+    d_st = torch.full((1,), -1, dtype=torch.int32, device="cuda")
+
+    def handle(solver):
+        monkeypatch.setenv("GFNFF_EEQ_SOLVER", solver)
+        g = GFNFF(precision=precision)
+        assert g.setMolecule(*_near_singular(0.74)), g.getErrorMessage()
+        assert g.eeqSolver() == solver
+        return g
+
+    def evaluate(g, bond):
+        d_x = torch.from_numpy(_near_singular(bond)[1] / 0.529177210903).cuda()
+        torch.cuda.synchronize()
+        assert lib.gfnff_energy_and_gradient_device(g.handle, d_x.data_ptr(), d_e.data_ptr(), None,
+                                                    d_st.data_ptr()) == 0
+        torch.cuda.synchronize()
+        return int(d_st[0]), float(d_e[0])
+
+    tiled, cg = handle("tiled"), handle("batched")
+    lo, hi = 0.471, 0.74
+    for _ in range(60):
+        mid = 0.5 * (lo + hi)
+        lo, hi = (lo, mid) if evaluate(tiled, mid)[0] == 0 else (mid, hi)
+    for d in (1e-11, 1e-10, 1e-9, 1e-8, 1e-6, 1e-4, 1e-2):
+        (s0, e0), (s1, e1) = evaluate(tiled, hi + d), evaluate(cg, hi + d)
+        assert (s0, s1) == (0, 0), (d, s0, s1)
+        assert abs(e1 - e0) < 1e-10 * e0 * e0 + 1e-9, (d, e0, e1)
+    for d in (1e-9, 1e-6, 1e-2):
+        assert evaluate(tiled, lo - d)[0] == evaluate(cg, lo - d)[0] == 3
