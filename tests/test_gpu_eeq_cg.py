@@ -173,3 +173,34 @@ def test_nearly_singular_matrix_on_the_device_entry(precision, monkeypatch):
         assert abs(e1 - e0) < 1e-10 * e0 * e0 + 1e-9, (d, e0, e1)
     for d in (1e-9, 1e-6, 1e-2):
         assert evaluate(tiled, lo - d)[0] == evaluate(cg, lo - d)[0] == 3
+
+
+def test_mixed_charges_end_far_below_the_bar(monkeypatch):
+    """The same right-hand sides solved by the FP64 Cholesky kernels: the recurrence ends at a residual
+    of 1e-14, so the charges agree to 1e-14 sqrt(n) / l_min < 2e-12 (n <= 300, smallest eigenvalue
+    >= 0.1); a solve that stops at the bar of 1e-10 is 1e-10 off."""
+    def perturbed(mols):
+        x = np.concatenate([x for _, x in mols])
+        return x + np.random.default_rng(1).normal(scale=0.03, size=x.shape)
+
+    for mols in (workloads.conformer_batch(24, 7), [workloads.water_cluster(k, k) for k in (3, 10, 30, 60)]):
+        q = []
+        for direct in (False, True):
+            monkeypatch.setenv("GFNFF_BATCH_TC", "0") if direct else monkeypatch.delenv("GFNFF_BATCH_TC", False)
+            g = GFNFF(precision=MIXED)
+            assert g.setMoleculeBatch(mols), g.getErrorMessage()
+            g.updateGeometry(perturbed(mols))
+            assert (g.calculateEnergyBatch()[1] == 0).all()
+            q.append(g.getCharges().copy())
+        assert np.abs(q[0] - q[1]).max() < 2e-12
+    for mol in (workloads.alkane(8, 8), workloads.alkane(100, 1)):
+        q = []
+        for solver in ("batched", "tiled"):
+            monkeypatch.setenv("GFNFF_EEQ_SOLVER", solver)
+            g = GFNFF(precision=MIXED)
+            assert g.setMolecule(*mol), g.getErrorMessage()
+            g.updateGeometry(perturbed([mol]))
+            g.calculateEnergy(True)
+            assert not g.hasError() and g.eeqSolver() == solver
+            q.append(g.getCharges().copy())
+        assert np.abs(q[0] - q[1]).max() < 2e-12
