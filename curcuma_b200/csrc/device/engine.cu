@@ -753,7 +753,7 @@ struct Engine::Impl {
     DBuf<int> pwarm;
     bool pcg_warm = false;
     // Molecules with fragments of more than 32 unknowns (chains): the block-Jacobi inverses
-    // come from the set-up geometry, computed once on the host (blocks up to 128 unknowns,
+    // come from the set-up geometry, computed once on the host (blocks up to 512 unknowns,
     // applied from global memory), instead of being recomputed in every launch from the
     // current matrix.  The preconditioner is then slightly stale, which costs iterations
     // only; the solve stays exact (GFNFF_PCG_PRE=0: off).
@@ -814,6 +814,7 @@ struct Engine::Impl {
         }
         A.binv_pre = pcg_pre ? pbinv.p : nullptr;
         A.big = pcg_big;
+        A.scratch = pcg_scratch(pcg_pre, pcg_lower);
         void* args[] = {&A};
         if (pcg_ir) {
             void* irargs[] = {&A, &pcg_tmap};
@@ -1741,7 +1742,8 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
                 if (const char* eb = std::getenv("GFNFF_PCG_PREBLK")) blkmax = std::max(2, std::min(512, std::atoi(eb)));
             }
         }
-        {
+        auto make_blocks = [&](int bmax) {
+            std::vector<int2> bl;
             int group = 0;
             if (const char* e = std::getenv("GFNFF_PCG_BLOCK")) group = std::max(0, std::min(kPcgWarpMax, std::atoi(e)));
             std::vector<int> fr(n);
@@ -1749,7 +1751,7 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
             for (int a = 0; a < n; ++a) fr[P.ix(0, a)] = M0.frag[a];
             int r = 0, i = 0, cur0 = 0, cur = 0;
             auto flush = [&]() {
-                if (cur > 0) blocks.push_back(make_int2(cur0, cur));
+                if (cur > 0) bl.push_back(make_int2(cur0, cur));
                 cur = 0;
             };
             while (i < n) {
@@ -1758,11 +1760,11 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
                 const int nr = j - i - 1;   // the fragment's anchor is its first atom
                 if (nr > group) {
                     flush();
-                    // equal chunks of at most blkmax
-                    const int nch = (nr + blkmax - 1) / blkmax, base = nr / nch, extra = nr % nch;
+                    // equal chunks of at most bmax
+                    const int nch = (nr + bmax - 1) / bmax, base = nr / nch, extra = nr % nch;
                     for (int c = 0, off = 0; c < nch; ++c) {
                         const int sz = base + (c < extra ? 1 : 0);
-                        blocks.push_back(make_int2(r + off, sz));
+                        bl.push_back(make_int2(r + off, sz));
                         off += sz;
                     }
                 } else if (nr > 0) {
@@ -1774,7 +1776,74 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
                 i = j;
             }
             flush();
-            if (r != P.nred) blocks.clear();   // fragments not contiguous: no PCG
+            if (r != P.nred) bl.clear();   // fragments not contiguous: no PCG
+            return bl;
+        };
+        // the lower-triangle form from 4096 unknowns (the matrix leaves L2), and for chains
+        // with set-up block inverses from 256: its tiled product balances work by tiles, so
+        // every SM takes part even where large preconditioner blocks, owned whole, would
+        // load a few blocks with most rows (Gly50 + 1500 waters: 1.45 -> 0.69 ms)
+        auto lower_form = [&]() {
+            const char* esym = std::getenv("GFNFF_PCG_SYM");
+            return esym ? std::strcmp(esym, "0") != 0 : (P.nred >= 4096 || (P.pcg_pre && P.nred >= 256));
+        };
+        // mixed form, lower-triangle systems: FP32-matrix CG inside FP64 refinement
+        // (k_pcg_ir; GFNFF_PCG_IR=0: the FP64 classic PCG at the absolute bar)
+        auto ir_form = [&]() {
+            const char* ef = std::getenv("GFNFF_PCG_F32");
+            const char* eir = std::getenv("GFNFF_PCG_IR");
+            return lower_form() && P.opt.precision == 1 && !(ef && !std::strcmp(ef, "1")) && !(eir && !std::strcmp(eir, "0"));
+        };
+        // rows per grid block (rows r0, r1, blocks b0, b1): whole preconditioner blocks, about
+        // nred / grid rows each, and the shared memory that this takes
+        struct PcgPlan {
+            std::vector<int4> part;
+            int maxrows = 1;
+            long long maxinv = 1;   // doubles of the owned inverses
+            size_t smem = 0, smem_ir = 0;
+        };
+        constexpr size_t kPcgSmemCap = 220 * 1024;
+        auto plan = [&](const std::vector<int2>& bl) {
+            PcgPlan pl;
+            std::vector<long long> boff{0};
+            for (auto& b : bl) boff.push_back(boff.back() + (long long)b.y * b.y);
+            const int G = lower_form() ? nsm : std::max(1, std::min(nsm, (int)bl.size()));
+            size_t bk = 0;
+            for (int g = 0; g < G; ++g) {
+                const int target = (int)(((long long)P.nred * (g + 1)) / G);
+                const int b0 = (int)bk, r0 = bk < bl.size() ? bl[bk].x : P.nred;
+                while (bk < bl.size() && (bl[bk].x + bl[bk].y <= target || g == G - 1)) ++bk;
+                const int r1 = bk < bl.size() ? bl[bk].x : P.nred;
+                pl.part.push_back(make_int4(r0, r1, b0, (int)bk));
+                pl.maxrows = std::max(pl.maxrows, r1 - r0);
+                pl.maxinv = std::max(pl.maxinv, boff[bk] - boff[b0]);
+            }
+            if (P.pcg_pre) pl.maxinv = 0;         // inverses applied from global memory
+            pl.maxinv = (pl.maxinv + 1) & ~1ll;   // keeps the int4 row records behind it 16-byte aligned
+            // p (n), scratch, x/r/z/Mp of the owned rows, owned block inverses
+            pl.smem = ((size_t)((P.nred + 1) & ~1) + pcg_scratch(P.pcg_pre, lower_form()) + 4 * (size_t)pl.maxrows + pl.maxinv) *
+                          sizeof(double) +
+                      (size_t)pl.maxrows * sizeof(int4);
+            // k_pcg_ir: one more owned-row vector (the inner correction d), even-sized, and the
+            // region of the replicated vector is the larger of the FP64 vector and the FP32
+            // direction with the staging halves of a tile
+            pl.smem_ir = pl.smem + (size_t)((pl.maxrows + 1) & ~1) * sizeof(double) +
+                         (size_t)(pcg_ir_pregion(P.nred) - ((P.nred + 1) & ~1)) * sizeof(double);
+            return pl;
+        };
+        blocks = make_blocks(blkmax);
+        // A grid block owns its preconditioner blocks whole, and their rows' vectors must fit beside the
+        // replicated one: smaller blocks only where whole fragments do not (fragments of 512
+        // unknowns: from 21,500 to 22,500 unknowns on), since a cut chain costs far more products (39
+        // C170H342, 19,929 unknowns: FP64 59 products, 33 ms, whole; 205, 102 ms, in blocks of 128).
+        if (P.pcg_pre) {
+            const int most = blkmax;
+            for (int bmax = most; bmax >= 128 || bmax == most; bmax /= 2) {
+                const std::vector<int2> bl = make_blocks(bmax);
+                if (plan(bl).smem > kPcgSmemCap) continue;
+                blocks = bl;
+                break;
+            }
         }
         if (!blocks.empty() && P.pcg_pre) {
             // set-up-geometry inverses of every block (host Cholesky), row-major like the
@@ -1826,8 +1895,6 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
             if (r != P.nred) blocks.clear();
         }
         if (!blocks.empty()) {
-            // rows per grid block: whole preconditioner blocks, about nred / nsm rows each
-            std::vector<int4> part;
             std::vector<long long> boff;
             long long bo = 0;
             P.pcg_big = false;
@@ -1836,38 +1903,16 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
                 bo += (long long)b.y * b.y;
                 P.pcg_big = P.pcg_big || b.y > kPcgRowThread;
             }
-            // the lower-triangle form from 4096 unknowns (the matrix leaves L2), and for chains
-            // with set-up block inverses from 256: its tiled product balances work by tiles, so
-            // every SM takes part even where large preconditioner blocks, owned whole, would
-            // load a few blocks with most rows (Gly50 + 1500 waters: 1.45 -> 0.69 ms)
-            const char* esym = std::getenv("GFNFF_PCG_SYM");
-            const bool lower = esym ? std::strcmp(esym, "0") != 0
-                                    : (P.nred >= 4096 || (P.pcg_pre && P.nred >= 256));
-            const int G = lower ? nsm : std::max(1, std::min(nsm, (int)blocks.size()));
-            size_t bk = 0;
-            int maxrows = 1;
-            long long maxinv = 1;
-            for (int g = 0; g < G; ++g) {
-                const int target = (int)(((long long)P.nred * (g + 1)) / G);
-                const int b0 = (int)bk, r0 = bk < blocks.size() ? blocks[bk].x : P.nred;
-                while (bk < blocks.size() && (blocks[bk].x + blocks[bk].y <= target || g == G - 1)) ++bk;
-                const int r1 = bk < blocks.size() ? blocks[bk].x : P.nred;
-                part.push_back(make_int4(r0, r1, b0, (int)bk));
-                maxrows = std::max(maxrows, r1 - r0);
-                maxinv = std::max(maxinv, (bk < blocks.size() ? boff[bk] : bo) - (b0 < (int)blocks.size() ? boff[b0] : bo));
-            }
-            // p (n), Gauss-Jordan scratch, x/r/z/Mp of the owned rows, owned block inverses
-            if (P.pcg_pre) maxinv = 0;      // inverses applied from global memory
-            maxinv = (maxinv + 1) & ~1ll;   // keeps the int4 row records behind it 16-byte aligned
-            const size_t smem =
-                ((size_t)((P.nred + 1) & ~1) + kPcgMaxBlock * (kPcgMaxBlock + 1) + 4 * (size_t)maxrows + maxinv) *
-                    sizeof(double) +
-                (size_t)maxrows * sizeof(int4);
-            if (smem <= 220 * 1024) {
+            const bool lower = lower_form();
+            const PcgPlan pl = plan(blocks);
+            const int G = (int)pl.part.size(), maxrows = pl.maxrows;
+            const long long maxinv = pl.maxinv;
+            const size_t smem = pl.smem;
+            if (smem <= kPcgSmemCap) {
                 std::vector<int> rblk(P.nred);
                 for (size_t q = 0; q < blocks.size(); ++q)
                     for (int r = 0; r < blocks[q].y; ++r) rblk[blocks[q].x + r] = (int)q;
-                P.pblocks.upload(blocks); P.pboff.upload(boff); P.ppart.upload(part); P.prblk.upload(rblk);
+                P.pblocks.upload(blocks); P.pboff.upload(boff); P.ppart.upload(pl.part); P.prblk.upload(rblk);
                 P.px.alloc(P.nred); P.pz.alloc(P.nred);
                 P.pcg_maxrows = maxrows;
                 P.pcg_maxinv = (int)maxinv;
@@ -1875,10 +1920,7 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
                     P.pcg_lower = lower;
                     const char* ef = std::getenv("GFNFF_PCG_F32");
                     P.pcg_f32 = P.pcg_lower && P.opt.precision == 1 && ef && !std::strcmp(ef, "1");
-                    // mixed form, lower-triangle systems: FP32-matrix CG inside FP64 refinement
-                    // (k_pcg_ir; GFNFF_PCG_IR=0: the FP64 classic PCG at the absolute bar)
-                    const char* eir = std::getenv("GFNFF_PCG_IR");
-                    P.pcg_ir = P.pcg_lower && P.opt.precision == 1 && !P.pcg_f32 && !(eir && !std::strcmp(eir, "0"));
+                    P.pcg_ir = ir_form();
                     if (P.pcg_f32 || P.pcg_ir) P.Mf.alloc((size_t)P.lda * P.nred);
                     if (P.pcg_ir) {
                         const size_t n4 = (size_t)((P.nred + 3) & ~3);
@@ -1907,14 +1949,11 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
                 int per_sm = 0;
                 CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_pcg, kPcgThreads, smem));
                 P.pcg_ready = per_sm >= 1;
-                if (P.pcg_ir) {   // one more owned-row vector (the inner correction d), even-sized
-                    // and the region of the replicated vector is the larger of the FP64 vector
-                    // and the FP32 direction with two staging halves of a tile
-                    P.pcg_smem_ir = smem + (size_t)((maxrows + 1) & ~1) * sizeof(double) +
-                                    (size_t)(pcg_ir_pregion(P.nred) - ((P.nred + 1) & ~1)) * sizeof(double);
+                if (P.pcg_ir) {
+                    P.pcg_smem_ir = pl.smem_ir;
                     int ps = 0;
                     const void* kir = (const void*)k_pcg_ir;
-                    if (P.pcg_smem_ir <= 220 * 1024) {
+                    if (P.pcg_smem_ir <= kPcgSmemCap) {
                         allow_smem(kir, P.pcg_smem_ir);
                         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, kir, kPcgThreads, P.pcg_smem_ir));
                     }
@@ -1926,7 +1965,7 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
                 // default: pipelined for L2-resident matrices (latency-bound); the tiled product
                 // of large ones measured faster in the classic form
                 P.pcg_pipe = pe ? std::strcmp(pe, "classic") != 0 : !P.pcg_lower;
-                P.pcg_pipe = P.pcg_pipe && P.pcg_smem_pipe <= 220 * 1024;
+                P.pcg_pipe = P.pcg_pipe && P.pcg_smem_pipe <= kPcgSmemCap;
                 {
                     const char* er = std::getenv("GFNFF_PCG_RES");
                     const int nt64 = (P.nred + 63) / 64;

@@ -46,6 +46,7 @@ struct PCGArgs {
                           // same system and is the initial guess; set to 1 on convergence
     const float* Mf;      // lower form in the mixed precision form: M stored in FP32 (M unused)
     bool big;             // there are preconditioner blocks of more than kPcgRowThread rows
+    int scratch;          // doubles of the scratch region G (pcg_scratch)
     const double* binv_pre;   // block inverses computed at set-up (global memory, boff layout), or null
     int lower;            // 1 or 2: only the lower triangle of M is stored; M p by tiles
                           // (matvec_tiles, streaming 4 or 8 columns per warp at once)
@@ -394,6 +395,13 @@ __device__ void take_tiles_result(const PCGArgs& A, int row0, int nrow, double* 
     __syncthreads();
 }
 
+// doubles of the scratch region: the row sums of a tile's warps, and a block under inversion
+// where the inverses are formed in the kernel (pcg_setup)
+__host__ __device__ constexpr int pcg_scratch(bool pre, bool lower)
+{
+    return pre && lower ? kPcgThreads / 32 * kPcgT : kPcgMaxBlock * (kPcgMaxBlock + 1);
+}
+
 // element accessor of the stored matrix (full, lower, or FP32 lower)
 struct MStored {
     const PCGArgs* A;
@@ -535,14 +543,13 @@ __device__ void pcg_setup(const PCGArgs& A, int4 pt, long long boff0, double* G,
 __global__ void __launch_bounds__(kPcgThreads) k_pcg(PCGArgs A)
 {
     extern __shared__ double sm[];
-    constexpr int GL = kPcgMaxBlock + 1;
     const int4 pt = A.part[blockIdx.x];
     const int row0 = pt.x, row1 = pt.y, nrow = row1 - row0;
     const long long boff0 = pt.z < pt.w ? A.boff[pt.z] : 0;
     double* p = sm;                              // n: search direction, replicated
-    double* G = p + ((A.n + 1) & ~1);            // kPcgMaxBlock x GL scratch (even offsets
-                                                 // keep the int4 records 16-byte aligned)
-    double* xs = G + kPcgMaxBlock * GL;          // owned rows: x, r, z, M p
+    double* G = p + ((A.n + 1) & ~1);            // scratch (even offsets keep the int4 records
+                                                 // 16-byte aligned)
+    double* xs = G + A.scratch;                  // owned rows: x, r, z, M p
     double* rs = xs + A.maxrows;
     double* zs = rs + A.maxrows;
     double* Ap = zs + A.maxrows;
@@ -878,15 +885,14 @@ __global__ void __launch_bounds__(kPcgThreads) k_pcg_ir(PCGArgs A, const __grid_
     }
     unsigned uses = 0;   // halves streamed through the ring (the stages' phases)
     bool tma_ok = true;
-    constexpr int GL = kPcgMaxBlock + 1;
     const int4 pt = A.part[blockIdx.x];
     const int row0 = pt.x, row1 = pt.y, nrow = row1 - row0;
     const long long boff0 = pt.z < pt.w ? A.boff[pt.z] : 0;
     double* p = sm;                              // n, replicated: x of the FP64 residual
     float* ring = reinterpret_cast<float*>(      // inner iterations: the tile staging ring
         (reinterpret_cast<size_t>(sm) + 127) & ~static_cast<size_t>(127));
-    double* G = p + pcg_ir_pregion(A.n);         // kPcgMaxBlock x GL scratch
-    double* xs = G + kPcgMaxBlock * GL;          // owned rows: x, r, z, M p, d
+    double* G = p + pcg_ir_pregion(A.n);         // scratch
+    double* xs = G + A.scratch;                  // owned rows: x, r, z, M p, d
     double* rs = xs + A.maxrows;
     double* zs = rs + A.maxrows;
     double* Ap = zs + A.maxrows;
@@ -1056,14 +1062,13 @@ __device__ void grid_totals3(const double* partial, int set, double& a, double& 
 __global__ void __launch_bounds__(kPcgPipeThreads, 2) k_pcg_pipe(PCGArgs A)
 {
     extern __shared__ double sm[];
-    constexpr int GL = kPcgMaxBlock + 1;
     const int4 pt = A.part[blockIdx.x];
     const int row0 = pt.x, row1 = pt.y, nrow = row1 - row0;
     const long long boff0 = pt.z < pt.w ? A.boff[pt.z] : 0;
     const int R = A.maxrows;
     double* v = sm;                              // n: operand of the next product, replicated
-    double* G = v + ((A.n + 1) & ~1);            // kPcgMaxBlock x GL scratch
-    double* xs = G + kPcgMaxBlock * GL;          // owned rows of x r u w z q s p m n
+    double* G = v + ((A.n + 1) & ~1);            // scratch
+    double* xs = G + A.scratch;                  // owned rows of x r u w z q s p m n
     double* rs = xs + R;
     double* us = rs + R;
     double* ws = us + R;
