@@ -753,7 +753,7 @@ struct Engine::Impl {
     DBuf<int> pwarm;
     bool pcg_warm = false;
     // Molecules with fragments of more than 32 unknowns (chains): the block-Jacobi inverses
-    // come from the set-up geometry, computed once on the host (blocks up to 512 unknowns,
+    // come from the set-up geometry, computed once (k_pcg_blkinv; blocks up to 512 unknowns,
     // applied from global memory), instead of being recomputed in every launch from the
     // current matrix.  The preconditioner is then slightly stale, which costs iterations
     // only; the solve stays exact (GFNFF_PCG_PRE=0: off).
@@ -1738,8 +1738,8 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
             const char* ep = std::getenv("GFNFF_PCG_PRE");
             P.pcg_pre = big > kPcgWarpMax && !(ep && !std::strcmp(ep, "0"));
             if (P.pcg_pre) {
-                blkmax = 512;   // whole fragments: 353 atoms in 1500 waters take 13 iterations, 47 in blocks of 128
-                if (const char* eb = std::getenv("GFNFF_PCG_PREBLK")) blkmax = std::max(2, std::min(512, std::atoi(eb)));
+                blkmax = kPcgPreMax;   // whole fragments: 353 atoms in 1500 waters take 13 iterations, 47 in blocks of 128
+                if (const char* eb = std::getenv("GFNFF_PCG_PREBLK")) blkmax = std::max(2, std::min(kPcgPreMax, std::atoi(eb)));
             }
         }
         auto make_blocks = [&](int bmax) {
@@ -1846,36 +1846,28 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
             }
         }
         if (!blocks.empty() && P.pcg_pre) {
-            // set-up-geometry inverses of every block (host Cholesky), row-major like the
-            // device-computed ones
-            auto A_el = [&](int a, int b) {
-                if (a == b) return adg[a];
-                const double dx = p0[a].x - p0[b].x, dy = p0[a].y - p0[b].y, dz = p0[a].z - p0[b].z;
-                const double d2 = dx * dx + dy * dy + dz * dz, sa = alp[a] + alp[b];
-                if (d2 >= 36.0 * sa) return 1.0 / std::sqrt(d2);
-                const double rr = std::sqrt(d2);
-                return std::erf(rr / std::sqrt(sa)) / rr;
-            };
-            std::vector<double> inv;
+            // set-up-geometry inverses of every block, row-major like those formed in the kernels
+            std::vector<long long> boff;
+            long long tot = 0;
             for (auto& b : blocks) {
-                const int sz = b.y;
-                std::vector<double> Mb((size_t)sz * sz), Ib((size_t)sz * sz, 0.0);
-                for (int i = 0; i < sz; ++i)
-                    for (int j = 0; j < sz; ++j) {
-                        const int k = P.h_r2a[b.x + i], ak = P.h_anchor[k];
-                        const int l = P.h_r2a[b.x + j], al = P.h_anchor[l];
-                        Mb[(size_t)i * sz + j] = A_el(k, l) - A_el(k, al) - A_el(ak, l) + A_el(ak, al);
-                    }
-                for (int i = 0; i < sz; ++i) Ib[(size_t)i * sz + i] = 1.0;
-                if (!linalg::cholesky(Mb.data(), sz)) {
-                    P.pcg_pre = false;   // not positive definite: inverses per launch instead
-                    break;
-                }
-                linalg::cholesky_solve(Mb.data(), sz, Ib.data(), sz);
-                inv.insert(inv.end(), Ib.begin(), Ib.end());
+                boff.push_back(tot);
+                tot += (long long)b.y * b.y;
             }
-            if (P.pcg_pre) P.pbinv.upload(inv);
-            else blocks.clear();   // rebuilt below with device-sized blocks
+            DBuf<int2> dblk;
+            DBuf<long long> doff;
+            DBuf<int> dbad;
+            dblk.upload(blocks);
+            doff.upload(boff);
+            dbad.upload(std::vector<int>{0});
+            P.pbinv.alloc((size_t)tot);
+            k_pcg_blkinv<<<(unsigned)blocks.size(), kPcgPreThreads, 0, P.stream>>>(P.view(), dblk.p, doff.p, P.red2atom.p,
+                                                                                  P.anchor.p, P.pbinv.p, dbad.p);
+            CK(cudaGetLastError());
+            CK(cudaStreamSynchronize(P.stream));
+            int bad = 0;
+            CK(cudaMemcpy(&bad, dbad.p, sizeof(int), cudaMemcpyDeviceToHost));
+            P.pcg_pre = !bad;      // not positive definite: inverses per launch instead
+            if (bad) blocks.clear();   // rebuilt below with device-sized blocks
         }
         if (blocks.empty() && !P.pcg_pre && blkmax != kPcgMaxBlock) {
             // the set-up inverses failed: fall back to per-fragment blocks of <= 64
