@@ -296,7 +296,7 @@ struct Engine::Impl {
     int n = 0, nfrag = 0, K = 0, nred = 0, nmol = 0, nsplit = 1;
     // Coulomb + D4 pairs: each pair once over a tile-pair list (default), or both
     // directions by rows (GFNFF_PAIRS=rows)
-    DBuf<int4> coul_tiles[3], d4_tiles[3];   // tile lists of k_pairs_coul and k_pairs_d4 per variant
+    DBuf<int4> coul_tiles[3], d4_tiles[3];   // tile lists of k_pairs_coul and k_pairs_d4 per variant (make_tiles)
     int n_coul_tiles[3] = {0, 0, 0}, n_d4_tiles[3] = {0, 0, 0};
     // CN neighbour list (k_cn_d4, k_tail): pairs within 6 + kCnSkin bohr of the
     // reference geometry cnl_ref, CSR by atom; cnl_bad = 1 once an atom moved more than
@@ -393,6 +393,43 @@ struct Engine::Impl {
     enum { PAIRS_SYM32 = 0, PAIRS_SYM64 = 1, PAIRS_SYM64_OCC = 2, PAIRS_ROWS = 3 };
     static constexpr int kCoulRows[3] = {32, 64, 128}, kD4Rows[3] = {32, 32, 32}, kPairCols[3] = {16, 32, 64};
     int pair_variant = PAIRS_SYM64;
+    // tiles of a variant: per molecule, row blocks from the molecule's first atom, their partners from the
+    // block's first row on; by increasing distance from the diagonal, so that the costlier near
+    // tiles (erf, exp, D4) start first.  One list for both kernels where their rows are the same
+    // (20,480 atoms: 0.4 million tiles, 6.6 MB, in the smallest variant, 0.07 million in the largest).
+    void make_tiles(int v)
+    {
+        if (v == PAIRS_ROWS || n_coul_tiles[v]) return;
+        int max_range = 0;
+        for (int m = 0; m < nmol; ++m) max_range = std::max(max_range, h_aoff[m + 1] - h_aoff[m]);
+        auto tiles = [&](int TR, int TC) {
+            std::vector<int4> tl;
+            for (int d = 0; d < max_range; d += TC)
+                for (int m = 0; m < nmol; ++m) {
+                    const int a0 = h_aoff[m], a1 = h_aoff[m + 1];
+                    for (int i0 = a0; i0 + d < a1; i0 += TR)
+                        tl.push_back(make_int4(i0, std::min(i0 + TR, a1), i0 + d, std::min(i0 + d + TC, a1)));
+                }
+            return tl;
+        };
+        const std::vector<int4> c = tiles(kCoulRows[v], kPairCols[v]);
+        coul_tiles[v].upload(c);
+        n_coul_tiles[v] = n_d4_tiles[v] = (int)c.size();
+        if (kD4Rows[v] == kCoulRows[v]) return;
+        const std::vector<int4> d = tiles(kD4Rows[v], kPairCols[v]);
+        d4_tiles[v].upload(d);
+        n_d4_tiles[v] = (int)d.size();
+    }
+    // the lists of every variant but `keep` go (PAIRS_ROWS: all)
+    void drop_tiles(int keep)
+    {
+        for (int v = 0; v < 3; ++v)
+            if (v != keep) {
+                coul_tiles[v].free();
+                d4_tiles[v].free();
+                n_coul_tiles[v] = n_d4_tiles[v] = 0;
+            }
+    }
     float pair_ms[4] = {-1.f, -1.f, -1.f, -1.f};   // the tuner's timings (ms per launch)
     // D4 pairs (charge-independent) on the side stream beside the EEQ solve, Coulomb pairs
     // after it on the main stream (GFNFF_PAIRS_SPLIT=0: both in one pass after the solve)
@@ -868,7 +905,7 @@ struct Engine::Impl {
     void launch_pairs_sym(int variant, const View& V, cudaStream_t st)
     {
         constexpr bool D4 = PART == kPairD4;
-        const int4* tl = (D4 ? d4_tiles : coul_tiles)[variant].p;
+        const int4* tl = (D4 && kD4Rows[variant] != kCoulRows[variant] ? d4_tiles : coul_tiles)[variant].p;
         const int nt = (D4 ? n_d4_tiles : n_coul_tiles)[variant];
         if (variant == PAIRS_SYM32) launch_pairs_tile<PART, 1, 16>(V, tl, nt, st);
         else if (variant == PAIRS_SYM64) launch_pairs_tile<PART, D4 ? 1 : 2, 32>(V, tl, nt, st);
@@ -1237,27 +1274,7 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
     int max_range = 0;
     for (int m = 0; m < nm; ++m) max_range = std::max(max_range, mols[m]->n);
     P.nsplit = pair_splits(n, max_range);
-    {   // tiles of k_pairs_coul / k_pairs_d4 per molecule: row blocks from the molecule's first atom, their
-        // partners from the block's first row on; by increasing distance from the diagonal, so
-        // that the costlier near tiles (erf, exp, D4) start first
-        auto tiles = [&](int TR, int TC) {
-            std::vector<int4> tl;
-            for (int d = 0; d < max_range; d += TC)
-                for (int m = 0; m < nm; ++m) {
-                    const int a0 = P.h_aoff[m], a1 = P.h_aoff[m + 1];
-                    for (int i0 = a0; i0 + d < a1; i0 += TR)
-                        tl.push_back(make_int4(i0, std::min(i0 + TR, a1), i0 + d, std::min(i0 + d + TC, a1)));
-                }
-            return tl;
-        };
-        for (int v = 0; v < 3; ++v) {
-            const std::vector<int4> c = tiles(Impl::kCoulRows[v], Impl::kPairCols[v]);
-            const std::vector<int4> d = tiles(Impl::kD4Rows[v], Impl::kPairCols[v]);
-            P.coul_tiles[v].upload(c);
-            P.d4_tiles[v].upload(d);
-            P.n_coul_tiles[v] = (int)c.size();
-            P.n_d4_tiles[v] = (int)d.size();
-        }
+    {
         const char* pe = std::getenv("GFNFF_PAIRS");
         P.pairs_sym = !(pe && !std::strcmp(pe, "rows"));
         const char* po = std::getenv("GFNFF_PAIRS_OCC");
@@ -1265,6 +1282,8 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
         // the variant before tuning
         P.pair_variant = !P.pairs_sym ? Impl::PAIRS_ROWS
                          : (nm > 1 ? Impl::PAIRS_SYM32 : (P.pairs_occ ? Impl::PAIRS_SYM64_OCC : Impl::PAIRS_SYM64));
+        P.drop_tiles(Impl::PAIRS_ROWS);   // of an earlier set-up of this handle
+        P.make_tiles(P.pair_variant);
         const char* ps = std::getenv("GFNFF_PAIRS_SPLIT");
         P.pairs_split = !ps ? 1 : (!std::strcmp(ps, "0") ? 0 : (!std::strcmp(ps, "1") ? 2 : 1));
     }
@@ -2107,6 +2126,8 @@ void Engine::tune_pairs(const std::vector<const Model*>& mols)
                 P.pair_variant = v;
                 P.pairs_sym = v != Impl::PAIRS_ROWS;
             }
+        P.make_tiles(P.pair_variant);
+        P.drop_tiles(P.pair_variant);
         return;
     }
     if ((et && !std::strcmp(et, "0")) || pe || po || P.n < 2) return;
@@ -2121,6 +2142,8 @@ void Engine::tune_pairs(const std::vector<const Model*>& mols)
         if (it != cache.end()) {
             P.pair_variant = it->second;
             P.pairs_sym = P.pair_variant != Impl::PAIRS_ROWS;
+            P.make_tiles(P.pair_variant);
+            P.drop_tiles(P.pair_variant);
             return;
         }
     }
@@ -2137,6 +2160,7 @@ void Engine::tune_pairs(const std::vector<const Model*>& mols)
     float best = 1e30f;
     int pick = P.pair_variant;
     for (int v = 0; v < 4; ++v) {
+        P.make_tiles(v);
         auto run = [&]() {
             if (v == Impl::PAIRS_ROWS) k_pairs<<<tgrid, kTile, 0, P.stream>>>(V, P.nsplit);
             else {
@@ -2162,6 +2186,7 @@ void Engine::tune_pairs(const std::vector<const Model*>& mols)
     cudaEventDestroy(e1);
     P.pair_variant = pick;
     P.pairs_sym = pick != Impl::PAIRS_ROWS;
+    P.drop_tiles(pick);
     std::lock_guard<std::mutex> lock(mu);
     cache[key] = pick;
 }

@@ -41,3 +41,25 @@ def test_variants_agree_and_tuner_picks_one(system, precision, monkeypatch):
         assert name == v
         assert np.abs(e - e0).max() < 1e-9, (v, e - e0)
         assert np.abs(g - g0).max() < 1e-9, v
+
+
+def test_only_the_lists_of_the_pick_are_kept(monkeypatch):
+    """14,739 atoms: the 32 x 16 tiles are 0.21 million, 3.4 MB; "rows" needs none.  The device's free memory
+    counts in steps of 2 MB."""
+    import torch
+
+    monkeypatch.setenv("GFNFF_EEQ_SOLVER", "pcg")
+    m = 17
+    site = 3.1 * np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), axis=-1).reshape(-1, 1, 3)
+    X = (site + workloads.water_geometry()[None]).reshape(-1, 3)
+    Z = np.tile(np.array([8, 1, 1], dtype=np.int32), m ** 3)
+    used = {}
+    for variant in ("rows", "rows", "sym32"):   # the first run also loads the kernels
+        monkeypatch.setenv("GFNFF_PAIRS_VARIANT", variant)
+        free0 = torch.cuda.mem_get_info()[0]
+        g = GFNFF(precision=FP64)
+        assert g.setMolecule(Z, X), g.getErrorMessage()
+        assert g.calculateEnergy(True) != 0.0
+        used[variant] = free0 - torch.cuda.mem_get_info()[0]
+        g.close()
+    assert used["sym32"] - used["rows"] >= 2 << 20, used
