@@ -38,6 +38,37 @@ __device__ __forceinline__ double eeq_a(const View& V, int a, int b)
     return erf(r / sqrt(s)) / r + born;
 }
 
+// Coordinates above 2^510 in absolute value (or not a number): squared distances may overflow, which
+// rsqrt_pos of the matrix builds does not take.  A build with such an atom takes its elements from
+// eeq_far, out of line (tested for and inlined at every element, the build of 14,440 unknowns took 0.54
+// instead of 0.45 ms).
+__device__ __forceinline__ bool far_coordinate(double x, double y, double z)
+{
+    const int hi = max(__double2hiint(x) & 0x7fffffff, max(__double2hiint(y) & 0x7fffffff, __double2hiint(z) & 0x7fffffff));
+    return hi >= (1023 + 510) << 20;
+}
+// entry of rows (k, ak), columns (l, al); pointers by value: a reference to the View would put a copy of it
+// on every thread's stack
+__device__ __noinline__ double eeq_far(const double4* pos, const double* alp, const double* adiag, const double* bdiag,
+                                       const double* brad, double keps, int4 id)
+{
+    const int a[4] = {id.x, id.x, id.y, id.y}, b[4] = {id.z, id.w, id.z, id.w};
+    double e[4];
+#pragma unroll 1
+    for (int t = 0; t < 4; ++t) {
+        const int i = a[t], j = b[t];
+        if (i == j) {
+            e[t] = adiag[i] + (brad ? bdiag[i] : 0.0);
+            continue;
+        }
+        const double4 pi = pos[i], pj = pos[j];
+        const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+        const double d2 = dx * dx + dy * dy + dz * dz, s = alp[i] + alp[j], r = sqrt(d2);
+        e[t] = (d2 >= 36.0 * s ? rsqrt(d2) : erf(r / sqrt(s)) / r) + (brad ? born_p16(keps, r, brad[i], brad[j]) : 0.0);
+    }
+    return e[0] - e[1] - e[2] + e[3];
+}
+
 // Reduced matrix by strips of 32 rows x COLS columns (a grid over strips and rows; strips above the
 // diagonal leave at once): the strip's row and column atoms and their anchors are staged in shared
 // memory, a warp takes COLS / 8 consecutive columns, its lanes the rows, and columns of one
@@ -60,6 +91,7 @@ __global__ void __launch_bounds__(256) k_eeq_M_tiles(View V, const int* __restri
     __shared__ double T[kMT][kMT + 1];
     const int r0 = blockIdx.y * kMT, c0 = blockIdx.x * COLS, n = V.nred;
     if (c0 > r0 + kMT - 1) return;
+    bool far = false;
     for (int t = threadIdx.x; t < 2 * (kMT + COLS); t += 256) {
         const bool row = t < 2 * kMT;
         const int u = row ? t : t - 2 * kMT, len = row ? kMT : COLS, w = u / len, i = u % len;
@@ -67,12 +99,13 @@ __global__ void __launch_bounds__(256) k_eeq_M_tiles(View V, const int* __restri
         int a = red2atom[idx];
         if (w) a = anchor[a];
         const double4 p = V.pos[a];
+        far |= far_coordinate(p.x, p.y, p.z);
         double* d = row ? &prow[w][0][i] : &pcol[w][0][i];
         d[0] = p.x; d[len] = p.y; d[2 * len] = p.z; d[3 * len] = V.alpeeq[a];
         if (BORN) d[4 * len] = V.brad[a];
         (row ? irow[w] : icol[w])[i] = a;
     }
-    __syncthreads();
+    far = __syncthreads_or(far);
     struct RowAtom {
         double x, y, z, h, al, br;
         int id;
@@ -109,7 +142,10 @@ __global__ void __launch_bounds__(256) k_eeq_M_tiles(View V, const int* __restri
                 ka = el(k, 1, cc);
                 aa = el(ak, 1, cc);
             }
-            const double v = el(k, 0, cc) - ka - el(ak, 0, cc) + aa;
+            double v = el(k, 0, cc) - ka - el(ak, 0, cc) + aa;
+            if (far)
+                v = eeq_far(V.pos, V.alpeeq, V.adiag, BORN ? V.bdiag : nullptr, BORN ? V.brad : nullptr, V.keps,
+                            make_int4(k.id, ak.id, icol[0][cc], icol[1][cc]));
             if (r < n && (full || r >= c)) {
                 M[(size_t)c * lda + r] = (TM)v;
                 if (M32) M32[(size_t)c * lda + r] = (float)v;

@@ -60,7 +60,8 @@ __host__ __device__ constexpr size_t cg_smem(int nr, int na, int cs)
 struct CgMol {
     double *x, *y, *z, *al, *ad, *br, *va;
     int *red, *anc;
-    bool single, born;
+    int a0;   // first atom of the molecule
+    bool single, born, far;
     double keps;
     __device__ double a(int i, int j) const
     {
@@ -73,9 +74,12 @@ struct CgMol {
         if (born) v += born_p16(keps, r, br[i], br[j]);
         return v;
     }
-    __device__ double m(int r, int c) const
+    __device__ __forceinline__ double m(const View& V, int r, int c) const
     {
         const int k = red[r], l = red[c];
+        if (far)
+            return eeq_far(V.pos, V.alpeeq, V.adiag, V.bdiag, V.brad, V.keps,
+                           make_int4(a0 + k, a0 + anc[r], a0 + l, a0 + anc[c]));
         if (single) return ((a(k, l) - va[r]) - va[c]) + ad[anc[r]];
         const int ak = anc[r], al_ = anc[c];
         return a(k, l) - a(k, al_) - a(ak, l) + a(ak, al_);
@@ -86,8 +90,10 @@ struct CgMol {
 __device__ void cg_stage(const View& V, const int* red2atom, const int* anchor, int r0, int nr, CgMol& S)
 {
     const int2 rg = V.jr[red2atom[r0]];
+    bool far = false;
     for (int i = threadIdx.x; i < rg.y - rg.x; i += blockDim.x) {
         const double4 p = V.pos[rg.x + i];
+        far |= far_coordinate(p.x, p.y, p.z);
         S.x[i] = p.x; S.y[i] = p.y; S.z[i] = p.z;
         S.al[i] = V.alpeeq[rg.x + i];
         S.ad[i] = V.adiag[rg.x + i] + (V.brad ? V.bdiag[rg.x + i] : 0.0);
@@ -101,7 +107,8 @@ __device__ void cg_stage(const View& V, const int* red2atom, const int* anchor, 
     S.single = anchor[red2atom[r0]] == anchor[red2atom[r0 + nr - 1]];
     S.born = V.brad != nullptr;
     S.keps = V.keps;
-    __syncthreads();
+    S.a0 = rg.x;
+    S.far = __syncthreads_or(far);
     if (S.single)
         for (int r = threadIdx.x; r < nr; r += blockDim.x) S.va[r] = S.a(S.red[r], S.anc[r]);
     __syncthreads();
@@ -314,13 +321,13 @@ __global__ void __launch_bounds__(kCgThreads) k_eeq_cg(View V, CgArgs A)
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
         if (CS == 1) {   // each element once, into both triangles
             for (int q = warp; q < rows; q += nw)
-                for (int c = lane; c <= q; c += 32) M[(size_t)q * nr + c] = M[(size_t)c * nr + q] = S.m(q, c);
+                for (int c = lane; c <= q; c += 32) M[(size_t)q * nr + c] = M[(size_t)c * nr + q] = S.m(V, q, c);
         } else {   // with M u, stored into every CTA once all of them run
             asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
             for (int q = warp; q < rows; q += nw) {
                 double g = 0.0;
                 for (int c = lane; c < nr; c += 32) {
-                    const double v = S.m(row0 + q, c);
+                    const double v = S.m(V, row0 + q, c);
                     M[(size_t)q * nr + c] = v;
                     g = fma(v, cg_start(c), g);
                 }
@@ -457,7 +464,7 @@ __global__ void __launch_bounds__(512) k_eeq_inv(View V, CgArgs A, float* pinv)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     for (int q = warp; q < rows; q += nw)
         for (int c = lane; c < nr; c += 32) {
-            const float v = (float)S.m(row0 + q, c);
+            const float v = (float)S.m(V, row0 + q, c);
             M[(size_t)q * ld + c] = v;
             if (c == row0 + q) diag[q] = v;
         }

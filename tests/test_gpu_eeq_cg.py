@@ -204,3 +204,36 @@ def test_mixed_charges_end_far_below_the_bar(monkeypatch):
             assert not g.hasError() and g.eeqSolver() == solver
             q.append(g.getCharges().copy())
         assert np.abs(q[0] - q[1]).max() < 2e-12
+
+
+@pytest.mark.parametrize("solver", ["tiled", "pcg", "batched"])
+def test_fragments_whose_squared_distance_overflows(solver, monkeypatch):
+    """Two flat waters, one 1e160 A away along its normal: no interaction, elements 1/r = 0.  Energy and
+    gradient are those at 1e6 A (device entry; the host entry would look for a new topology)."""
+    import torch
+
+    w = workloads.water_geometry()
+    w = w - w[0]
+    flat = np.stack([np.zeros(3), w[:, 0], w[:, 1]], axis=1)
+
+    def waters(dx):
+        return np.concatenate([flat, flat + np.array([dx, 0.0, 0.0])])
+
+    monkeypatch.setenv("GFNFF_EEQ_SOLVER", solver)
+    g = GFNFF(precision=FP64)
+    assert g.setMolecule(np.array([8, 1, 1, 8, 1, 1], dtype=np.int32), waters(4.0)), g.getErrorMessage()
+    assert g.eeqSolver() == solver
+    out = []
+    for dx in (1e6, 1e160):
+        d_x = torch.from_numpy(waters(dx) / 0.529177210903).cuda()
+        d_e = torch.zeros(1, dtype=torch.float64, device="cuda")
+        d_g = torch.zeros(d_x.shape, dtype=torch.float64, device="cuda")
+        d_st = torch.full((1,), -1, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        assert _lib.load().gfnff_energy_and_gradient_device(g.handle, d_x.data_ptr(), d_e.data_ptr(), d_g.data_ptr(),
+                                                            d_st.data_ptr()) == 0
+        torch.cuda.synchronize()
+        assert int(d_st[0]) == 0
+        out.append((float(d_e[0]), d_g.cpu().numpy()))
+    assert abs(out[0][0] - out[1][0]) < 1e-6    # 1 / (1e6 A) per pair of charges at most
+    assert np.abs(out[0][1] - out[1][1]).max() < 1e-6
