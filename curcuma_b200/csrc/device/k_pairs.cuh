@@ -165,10 +165,11 @@ __device__ __forceinline__ bool tile_far(const View& V, int r0, int r1, int j0, 
     float gap2 = 0.f;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        const float rl = (float)__reduce_min_sync(full, __double2int_rd(16.0 * px[d]));
-        const float rh = (float)__reduce_max_sync(full, __double2int_ru(16.0 * px[d]));
-        const float cl = (float)__reduce_min_sync(full, clo[d]), ch = (float)__reduce_max_sync(full, chi[d]);
-        const float gap = fmaxf(0.f, fmaxf(cl - rh, rl - ch));
+        const long long rl = __reduce_min_sync(full, __double2int_rd(16.0 * px[d]));
+        const long long rh = __reduce_max_sync(full, __double2int_ru(16.0 * px[d]));
+        const long long cl = __reduce_min_sync(full, clo[d]), ch = __reduce_max_sync(full, chi[d]);
+        // integers up to the difference: a coordinate of 1e8 bohr in FP32 is 8 bohr off
+        const float gap = (float)max(0ll, max(cl - rh, rl - ch));
         gap2 += gap * gap;
     }
     return gap2 > cut2 * 256.f * 1.0001f;

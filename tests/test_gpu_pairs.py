@@ -8,7 +8,7 @@ energies by its square and the gradient by about 1e-12."""
 import numpy as np
 import pytest
 
-from curcuma_b200 import FP64, GFNFF, workloads
+from curcuma_b200 import FP64, GFNFF, _lib, workloads
 from tests.oracle_api import Oracle
 
 pytestmark = pytest.mark.gpu
@@ -66,3 +66,32 @@ def test_batch_of_ragged_molecules(monkeypatch):
             T, Go, q, cn = Oracle(Z, X).engrad(X)
             assert abs(em - T["total"]) < 1e-10
             assert np.abs(gm - Go).max() < 1e-10
+
+
+def test_tiles_far_from_the_origin(monkeypatch):
+    """800 bohr of waters (tiles of every distance) translated to 5e7 and 1e8 bohr: the tile kernels leave
+    out no pair that the row kernel has.  Same coordinates, same charges: the energies (-130 Eh) differ
+    by the order of summation, some 1e-11; the pairs that FP32 box gaps lose are 4e-10 to 1e-9."""
+    import torch
+
+    w = workloads.water_geometry()
+    w = w - w[0]
+    X = np.concatenate([w + 3.1 * np.array([k // 4, k % 4 // 2, k % 2]) for k in range(400)])
+    Z = np.tile(np.array([8, 1, 1], dtype=np.int32), 400)
+    lib = _lib.load()
+    out = {}
+    for variant in ["rows"] + VARIANTS:
+        monkeypatch.setenv("GFNFF_PAIRS_VARIANT", variant)
+        g = GFNFF(precision=FP64)
+        assert g.setMolecule(Z, X), g.getErrorMessage()
+        for shift in (3e7, 6e7):
+            d_x = torch.from_numpy((X + shift) / 0.529177210903).cuda()
+            d_e = torch.zeros(1, dtype=torch.float64, device="cuda")
+            d_st = torch.full((1,), -1, dtype=torch.int32, device="cuda")
+            torch.cuda.synchronize()
+            assert lib.gfnff_energy_and_gradient_device(g.handle, d_x.data_ptr(), d_e.data_ptr(), None,
+                                                        d_st.data_ptr()) == 0
+            torch.cuda.synchronize()
+            assert int(d_st[0]) == 0
+            out[variant, shift] = float(d_e[0])
+            assert abs(out[variant, shift] - out["rows", shift]) < 1e-10, (variant, shift)
