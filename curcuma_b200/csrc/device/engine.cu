@@ -49,6 +49,7 @@
 namespace gfnff {
 
 #include "common.cuh"
+#include "recip.cuh"
 #include "k_bonded.cuh"
 #include "k_nonbonded.cuh"
 #include "k_pairs.cuh"

@@ -26,7 +26,8 @@
 // negative axis), and symmetric molecules have right-hand sides without one (H2: b = 0).  So the
 // solve starts from a pseudo-random vector u (cg_start), scaled so that M u is an eighth of b: every
 // direction is in the first residual, whatever b is.  M u comes out of the build of M (with it and
-// the larger first residual, 193 unknowns at 18 products: 77.0 -> 79.3 us; the counts are the same).
+// the larger first residual, 193 unknowns at 14 products: 65 -> 69 us, 25 unknowns the same; the counts
+// do not change).
 #pragma once
 
 namespace {
@@ -74,12 +75,15 @@ struct CgMol {
         if (born) v += born_p16(keps, r, br[i], br[j]);
         return v;
     }
-    __device__ __forceinline__ double m(const View& V, int r, int c) const
+    // `far` molecules: out of line, from the atoms in global memory
+    __device__ double m_far(const View& V, int r, int c) const
+    {
+        return eeq_far(V.pos, V.alpeeq, V.adiag, V.bdiag, V.brad, V.keps,
+                       make_int4(a0 + red[r], a0 + anc[r], a0 + red[c], a0 + anc[c]));
+    }
+    __device__ double m(int r, int c) const
     {
         const int k = red[r], l = red[c];
-        if (far)
-            return eeq_far(V.pos, V.alpeeq, V.adiag, V.bdiag, V.brad, V.keps,
-                           make_int4(a0 + k, a0 + anc[r], a0 + l, a0 + anc[c]));
         if (single) return ((a(k, l) - va[r]) - va[c]) + ad[anc[r]];
         const int ak = anc[r], al_ = anc[c];
         return a(k, l) - a(k, al_) - a(ak, l) + a(ak, al_);
@@ -211,12 +215,16 @@ __device__ __forceinline__ void cg_dots(const double* r, const double* z, const 
     rmax = __uint_as_float(__reduce_max_sync(full, m));
 }
 
-// max |v|, the same in every warp
-__device__ __forceinline__ float cg_max(const double* v, int n)
+// max |v| and max |w|, the same in every warp
+__device__ __forceinline__ void cg_max(const double* v, const double* w, int n, float& vmax, float& wmax)
 {
-    unsigned m = 0;
-    for (int c = threadIdx.x & 31; c < n; c += 32) m = max(m, abs_bits(v[c]));
-    return __uint_as_float(__reduce_max_sync(0xffffffffu, m));
+    unsigned a = 0, b = 0;
+    for (int c = threadIdx.x & 31; c < n; c += 32) {
+        a = max(a, abs_bits(v[c]));
+        b = max(b, abs_bits(w[c]));
+    }
+    vmax = __uint_as_float(__reduce_max_sync(0xffffffffu, a));
+    wmax = __uint_as_float(__reduce_max_sync(0xffffffffu, b));
 }
 
 // entry c of the start vector, in [-1, 1): the bits of c mixed by multiplications and shifts
@@ -316,31 +324,35 @@ __global__ void __launch_bounds__(kCgThreads) k_eeq_cg(View V, CgArgs A)
             bulk_copy(cg_raw, A.pinv + A.poff[mol] + (size_t)row0 * ld, bytes, &bar);
         }
     }
+    for (int q = threadIdx.x; q < nr; q += blockDim.x) x[q] = cg_start(q);
     cg_stage(V, A.red2atom, A.anchor, r0, nr, S);
     {
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-        if (CS == 1) {   // each element once, into both triangles
-            for (int q = warp; q < rows; q += nw)
-                for (int c = lane; c <= q; c += 32) M[(size_t)q * nr + c] = M[(size_t)c * nr + q] = S.m(V, q, c);
-        } else {   // with M u, stored into every CTA once all of them run
-            asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        // M u of the slice is stored into every CTA once all of them run
+        if (CS > 1) asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        auto build = [&](auto el) {
             for (int q = warp; q < rows; q += nw) {
+                if (CS == 1) {   // each element once, into both triangles
+                    for (int c = lane; c <= q; c += 32) M[(size_t)q * nr + c] = M[(size_t)c * nr + q] = el(q, c);
+                    continue;
+                }
                 double g = 0.0;
                 for (int c = lane; c < nr; c += 32) {
-                    const double v = S.m(V, row0 + q, c);
+                    const double v = el(row0 + q, c);
                     M[(size_t)q * nr + c] = v;
-                    g = fma(v, cg_start(c), g);
+                    g = fma(v, x[c], g);
                 }
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
                 if (lane < CS) cluster_store(w + row0 + q, lane, g);
             }
-        }
+        };
+        if (S.far) build([&](int r, int c) { return S.m_far(V, r, c); });
+        else build([&](int r, int c) { return S.m(r, c); });
     }
     for (int q = threadIdx.x; q < nr; q += blockDim.x) {
         const int k = A.red2atom[r0 + q];
         b[q] = eeq_rhs_atom(V, k, A.qlist, A.nq, A.q0) - eeq_rhs_atom(V, A.anchor[k], A.qlist, A.nq, A.q0);
-        x[q] = cg_start(q);
     }
     if (rows > 0) mbar_wait(&bar, 0);   // bounded; without the inverse the solve fails its checks
     cluster_barrier<CS>();
@@ -348,12 +360,12 @@ __global__ void __launch_bounds__(kCgThreads) k_eeq_cg(View V, CgArgs A)
         cg_product<CS, double>(M, nr, rows, row0, nr, x, w);
         __syncthreads();
     }
-    const float bmax = cg_max(b, nr), umax = cg_max(w, nr);
+    float bmax, umax;
+    cg_max(b, w, nr, bmax, umax);
     {
         // (mixed form: at least 1e-4 where b is smaller than that, far above the residual to reach)
         const float size = A.tol_abs > 0.0 ? fmaxf(bmax, 1e7f * (float)A.tol_abs) : bmax;
-        const double t = size > 0.f ? 0.125 * (double)size / (double)umax : 1.0;
-        __syncthreads();   // x read by the product
+        const double t = size > 0.f ? (double)(0.125f * size / umax) : 1.0;
         for (int q = threadIdx.x; q < nr; q += blockDim.x) {
             x[q] *= t;
             r[q] = b[q] - t * w[q];
@@ -366,7 +378,7 @@ __global__ void __launch_bounds__(kCgThreads) k_eeq_cg(View V, CgArgs A)
     // from one pass over r, z and w = M z; M p is carried along as s.  A CTA stores its slice of the
     // next z while another may still read the last one, so z alternates between two buffers; w is
     // stored only after the barrier that follows z, which every CTA reaches with its reads done.
-    double rz, zw, rz_old = 0.0, alpha = 0.0, dummy;
+    double rz, zw, irz_old = 0.0, ialpha = 0.0, dummy;   // 1 / the last r.z and alpha
     float rmax;
     const float scale = bmax > 0.f ? bmax : umax;
     const float stop = A.tol_abs > 0.0 ? 1e-4f * (float)A.tol_abs : 1e-15f * scale;
@@ -397,14 +409,15 @@ __global__ void __launch_bounds__(kCgThreads) k_eeq_cg(View V, CgArgs A)
             start = true;
             continue;
         }
-        const double beta = start ? 0.0 : rz * rcp_pos(rz_old);
-        const double pmp = start ? zw : zw - beta * rz * rcp_pos(alpha);
+        const double beta = start ? 0.0 : rz * irz_old;
+        const double pmp = start ? zw : zw - beta * rz * ialpha;
         if (!(pmp > 0.0 && rz > 0.0)) {   // not positive definite, or not a number
             state = 1;
             break;
         }
-        alpha = rz * rcp_pos(pmp);
-        rz_old = rz;
+        const double alpha = rz / pmp;
+        irz_old = 1.0 / rz;
+        ialpha = pmp * irz_old;
         __syncthreads();   // every warp has read r, z and w
         for (int q = threadIdx.x; q < nr; q += blockDim.x) {
             const double pq = start ? z[q] : z[q] + beta * p[q], sq = start ? w[q] : w[q] + beta * s[q];
@@ -464,7 +477,7 @@ __global__ void __launch_bounds__(512) k_eeq_inv(View V, CgArgs A, float* pinv)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     for (int q = warp; q < rows; q += nw)
         for (int c = lane; c < nr; c += 32) {
-            const float v = (float)S.m(V, row0 + q, c);
+            const float v = (float)S.m(row0 + q, c);
             M[(size_t)q * ld + c] = v;
             if (c == row0 + q) diag[q] = v;
         }

@@ -28,26 +28,6 @@ namespace {
 // at 128 registers spilled and measured 3 % slower on the 20,480-atom cluster)
 constexpr int kPairWarps = 12;
 
-// 1/sqrt(x) of a normal positive x: the hardware's ~20-bit estimate and one third-order step
-// y (1 + e/2 + 3/8 e^2), e = 1 - x y^2 (the series of (1 - e)^(-1/2)); within 1.3 ulp over 1e-9
-// .. 1e26 (measured), where the library call adds its special cases
-__device__ __forceinline__ double rsqrt_pos(double x)
-{
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-(x * y), y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
-// 1/x of a normal positive x: estimate and one third-order step y (1 + e + e^2), e = 1 - x y
-__device__ __forceinline__ double rcp_pos(double x)
-{
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y, 1.0);
-    return fma(y, fma(e, e, e), y);
-}
-
 // c += A B, A 16 x 4 (lane: rows g and g + 8, column t), B 4 x 8 (lane: row t, column g),
 // c 16 x 8 (lane: rows g, g, g + 8, g + 8, columns 2t, 2t + 1, 2t, 2t + 1)
 __device__ __forceinline__ void mma_16x8x4(double (&c)[4], double a0, double a1, double b)

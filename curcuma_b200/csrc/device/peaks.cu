@@ -1,9 +1,12 @@
-// Arithmetic-peak microbenchmarks: the roofline denominators for the FP64 / FP32 SIMT
-// kernels (the HBM and bf16 tensor peaks come from the pool's own measurement).
-// Each thread runs 8 independent FMA chains; the grid fills every SM several times.
+// Arithmetic diagnostics.  Peak microbenchmarks: the roofline denominators for the FP64 / FP32 SIMT
+// kernels; each thread runs 8 independent FMA chains; the grid fills every SM several times.
+// And the accuracy of the reciprocals of recip.cuh.
 #include <cuda_runtime.h>
 
+#include <cmath>
+
 #include "../../../include/gfnff_b200.h"
+#include "recip.cuh"
 
 namespace {
 
@@ -51,7 +54,39 @@ double run(int device)
     return cudaGetLastError() == cudaSuccess ? best : -1.0;
 }
 
+// largest difference from the library function over n arguments, spread evenly over log [lo, hi] with
+// their low bits mixed, in units in the last place of the library's result
+__global__ void k_recip_ulps(int root, double loglo, double step, long n, double* worst)
+{
+    double m = 0.0;
+    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
+        unsigned h = (unsigned)k * 2654435761u;
+        h ^= h >> 15;
+        const double x0 = exp(loglo + step * (double)k);
+        const double x = __hiloint2double(__double2hiint(x0), (int)(h * 2246822519u));
+        const double ref = root ? rsqrt(x) : 1.0 / x, got = root ? rsqrt_pos(x) : rcp_pos(x);
+        const double ulp = scalbn(1.0, ilogb(ref) - 52);
+        const double d = fabs(got - ref) / ulp;
+        m = d > m || !(d == d) ? d : m;
+        if (!(d == d)) break;
+    }
+    // non-negative doubles (and NaN, above them) order like their bits
+    atomicMax(reinterpret_cast<unsigned long long*>(worst), (unsigned long long)__double_as_longlong(m) & 0x7fffffffffffffffull);
+}
+
 }  // namespace
+
+extern "C" double gfnff_reciprocal_ulps(int device, int root, double lo, double hi, long n)
+{
+    if (!(lo > 0.0) || !(hi >= lo) || n < 2 || cudaSetDevice(device) != cudaSuccess) return -1.0;
+    double *d = nullptr, h = -1.0;
+    if (cudaMalloc(&d, sizeof(double)) != cudaSuccess) return -1.0;
+    cudaMemset(d, 0, sizeof(double));
+    k_recip_ulps<<<1184, 256>>>(root, std::log(lo), (std::log(hi) - std::log(lo)) / (double)(n - 1), n, d);
+    if (cudaMemcpy(&h, d, sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess) h = -1.0;
+    cudaFree(d);
+    return h;
+}
 
 extern "C" double gfnff_fma_peak_tflops(int device, int fp64)
 {

@@ -200,6 +200,11 @@ int gfnff_phase_times(gfnff_handle* h, double* ms, int cap);
  * counterpart in the reference. */
 double gfnff_fma_peak_tflops(int device, int fp64);
 
+/* Largest difference, in units in the last place, between the reciprocal (root != 0: reciprocal square root)
+ * that the pair and EEQ matrix kernels use and CUDA's, over n arguments spread over [lo, hi]; -1 on
+ * an error.  Diagnostic without a counterpart in the reference. */
+double gfnff_reciprocal_ulps(int device, int root, double lo, double hi, long n);
+
 /* Allocation-free EEQ charges, for callers that cannot allocate device memory (code
  * running inside another framework's memory pool, loops that forbid allocations after
  * start-up).  No counterpart in the reference.  Every buffer is a device pointer owned
