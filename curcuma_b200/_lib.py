@@ -24,7 +24,7 @@ EXPORTED = ["gfnff_default_options", "gfnff_create", "gfnff_setup", "gfnff_energ
             "gfnff_energy_and_gradient_batch", "gfnff_md_nve", "gfnff_kernels_per_evaluation",
             "gfnff_save_parameters", "gfnff_setup_from_parameters", "gfnff_write_parameters",
             "gfnff_pair_kernel", "gfnff_eeq_fp64_products", "gfnff_set_solvent", "gfnff_set_geometry_file",
-            "gfnff_topology_cache_hit", "gfnff_write_topology_cache", "gfnff_set_unit_cell", "gfnff_reciprocal_ulps"]
+            "gfnff_topology_cache_hit", "gfnff_write_topology_cache", "gfnff_set_unit_cell", "gfnff_reciprocal_ulps", "gfnff_batch_kernel"]
 PHASES = ["positions", "cn", "d4_weights", "eeq_matrix", "eeq_rhs", "eeq_solve", "bonded",
           "hbonds", "repulsion", "pairs", "post_chain", "finish"]
 
@@ -73,6 +73,8 @@ def load():
     lib.gfnff_eeq_solver.restype = ctypes.c_char_p
     lib.gfnff_pair_kernel.argtypes = [c_v]
     lib.gfnff_pair_kernel.restype = ctypes.c_char_p
+    lib.gfnff_batch_kernel.argtypes = [c_v]
+    lib.gfnff_batch_kernel.restype = ctypes.c_char_p
     lib.gfnff_eeq_iterations.argtypes = [c_v]
     lib.gfnff_eeq_fp64_products.argtypes = [c_v]
     lib.gfnff_set_solvent.argtypes = [c_v, ctypes.c_char_p]
@@ -89,7 +91,7 @@ def load():
     lib.gfnff_md_nve.argtypes = [c_v, c_i, c_d, P(c_d), P(c_d), P(c_d), P(c_d), P(c_d)]
     for name in EXPORTED:
         if name not in ("gfnff_default_options", "gfnff_stream", "gfnff_last_error", "gfnff_fma_peak_tflops", "gfnff_reciprocal_ulps",
-                        "gfnff_eeq_solver", "gfnff_pair_kernel"):
+                        "gfnff_eeq_solver", "gfnff_pair_kernel", "gfnff_batch_kernel"):
             getattr(lib, name).restype = c_i
     _lib = lib
     return lib

@@ -665,6 +665,12 @@ const char* gfnff_pair_kernel(gfnff_handle* h)
     return h->eng->pair_kernel_name();
 }
 
+const char* gfnff_batch_kernel(gfnff_handle* h)
+{
+    if (!h || !h->ready) return "";
+    return h->eng->batch_kernel_name();
+}
+
 int gfnff_kernels_per_evaluation(gfnff_handle* h)
 {
     if (!h || !h->ready) return -1;

@@ -484,7 +484,7 @@ struct Engine::Impl {
     std::vector<cudaEvent_t> cg_done;
     cudaEvent_t cg_fork = nullptr;
     // bins of the molecules with nr unknowns and na atoms each
-    void plan_cg(const std::vector<int>& nr, const std::vector<int>& na)
+    void plan_cg(const std::vector<int>& nr, const std::vector<int>& na, bool any_size)
     {
         cg_bins.clear();
         const size_t cap = 208 * 1024;
@@ -502,7 +502,7 @@ struct Engine::Impl {
             ctas += cs[m];
             slots += cs[m] > 1 ? cs[m] : std::max(1.0 / 8.0, cg_smem(nr[m], na[m], 1) / 222e3);
         }
-        if (slots > waves * 148.0) return;
+        if (!any_size && slots > waves * 148.0) return;
         // few molecules: larger clusters while the SMs hold one CTA each (a product and the
         // build shrink with the slice; below ~48 unknowns the barriers cost more)
         for (int top = 2; top <= 4; top *= 2) {
@@ -1436,15 +1436,17 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
         // (a candidate EEQ solver for them)
         P.batch_ready = nm > 1 || n <= kStageAtoms;
         P.cg_on = false;
+        // GFNFF_BATCH_CG=0: no conjugate gradients, 1: whatever the size of the batch;
         // GFNFF_BATCH_TC=0: the FP64 Cholesky for every molecule
-        const char* ecg = std::getenv("GFNFF_BATCH_TC");
-        if (P.batch_ready && P.nred > 0 && !(ecg && !std::strcmp(ecg, "0"))) {
+        const char* ecg = std::getenv("GFNFF_BATCH_CG");
+        const char* etc0 = std::getenv("GFNFF_BATCH_TC");
+        if (P.batch_ready && P.nred > 0 && !(ecg && !std::strcmp(ecg, "0")) && !(etc0 && !std::strcmp(etc0, "0"))) {
             std::vector<int> nr(nm), na(nm);
             for (int m = 0; m < nm; ++m) {
                 nr[m] = roff[m + 1] - roff[m];
                 na[m] = mols[m]->n;
             }
-            P.plan_cg(nr, na);
+            P.plan_cg(nr, na, ecg && !std::strcmp(ecg, "1"));
         }
         if (P.batch_ready) {
             std::vector<int> ord(nm);
@@ -2190,6 +2192,12 @@ void Engine::tune_pairs(const std::vector<const Model*>& mols)
     P.drop_tiles(pick);
     std::lock_guard<std::mutex> lock(mu);
     cache[key] = pick;
+}
+
+const char* Engine::batch_kernel_name() const
+{
+    if (!p_->batch_ready || (p_->nmol == 1 && (p_->use_lu || p_->solver != Impl::SOLVE_BATCH))) return "";
+    return p_->cg_on ? "cg" : (p_->batch_tc ? "tensor" : "cholesky");
 }
 
 const char* Engine::pair_kernel_name() const

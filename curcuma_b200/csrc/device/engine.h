@@ -94,6 +94,7 @@ public:
     // Coulomb + D4 pair kernel variant picked by the set-up autotuner: "sym32", "sym64",
     // "sym64_occ10" or "rows"
     const char* pair_kernel_name() const;
+    const char* batch_kernel_name() const;
     // iterations of the last iterative EEQ solve (0 for direct solvers)
     int eeq_iterations();
     // k_pcg_ir: FP64 products with the reduced matrix in the last solve; -1 otherwise

@@ -328,6 +328,10 @@ class GFNFF:
         """Pair kernel variant picked by the set-up autotuner (diagnostic)."""
         return self._lib.gfnff_pair_kernel(self._h).decode()
 
+    def batchKernel(self) -> str:
+        """How the charges of a batch are solved: "cg", "tensor" or "cholesky" """
+        return self._lib.gfnff_batch_kernel(self._h).decode()
+
     def eeqSolver(self) -> str:
         """EEQ solver chosen at setup ("library", "tiled", "pcg", "lu", "batched")."""
         return self._lib.gfnff_eeq_solver(self._h).decode()

@@ -247,6 +247,14 @@ const char* gfnff_eeq_solver(gfnff_handle* h);
  * counterpart in the reference. */
 const char* gfnff_pair_kernel(gfnff_handle* h);
 
+/* How the charges of a batch (or of a single molecule whose solver is "batched") are solved: "cg"
+ * (conjugate gradients with the set-up inverses), "tensor" (mixed form: FP32 Cholesky on the
+ * tensor cores with FP64 refinement) or "cholesky" (FP64 Cholesky); "" before setup and for the other
+ * solvers.  Chosen by the size of the batch; GFNFF_BATCH_CG=0|1 turns conjugate gradients off or on for
+ * every size, GFNFF_BATCH_TC=0 asks for the FP64 Cholesky.  Diagnostic without a counterpart in the
+ * reference. */
+const char* gfnff_batch_kernel(gfnff_handle* h);
+
 /* Iterations of the last iterative EEQ solve (0 for the direct solvers, -1 before
  * setup); synchronises the handle's stream.  Diagnostic without a counterpart in the
  * reference. */

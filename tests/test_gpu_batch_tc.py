@@ -12,6 +12,13 @@ from tests.oracle_api import Oracle, golden
 
 pytestmark = pytest.mark.gpu
 
+
+@pytest.fixture(autouse=True)
+def no_conjugate_gradients(monkeypatch):
+    """Batches of this size go to conjugate gradients by themselves"""
+    monkeypatch.setenv("GFNFF_BATCH_CG", "0")
+
+
 E_TOL = 1e-6
 G_TOL = 1e-5
 Q_TOL = 1e-8   # same system: ||M dy||_inf <= 1e-10, lambda_min(M) >= 0.1, n <= 300
@@ -51,6 +58,7 @@ def test_batch_tc_against_oracle_and_fp64(monkeypatch):
     ea, sa = a.calculateEnergyBatch()
     eb, sb = b.calculateEnergyBatch()
     assert (sa == 0).all() and (sb == 0).all(), (sa, sb)
+    assert (a.batchKernel(), b.batchKernel()) == ("cholesky", "tensor")
     it = b.eeqIterations()
     assert 1 <= it <= 8, it   # refinement corrections of the slowest molecule
     assert np.abs(a.getCharges() - b.getCharges()).max() < Q_TOL
@@ -71,6 +79,7 @@ def test_batch_tc_repeated_and_charged():
     charges = [0] * 6 + [1]
     b = GFNFF(precision=MIXED)
     assert b.setMoleculeBatch(mols, charges), b.getErrorMessage()
+    assert b.batchKernel() == "tensor"
     e1, s1 = b.calculateEnergyBatch()
     q1 = b.getCharges().copy()
     e2, s2 = b.calculateEnergyBatch()
@@ -84,13 +93,12 @@ def test_batch_tc_repeated_and_charged():
 
 
 def test_single_molecule_tc_solver(monkeypatch):
-    """A single molecule of the mixed form through the batched solver (the path a 194-atom
-    alkane takes when the autotuner picks it)."""
+    """A single molecule of the mixed form through the batched solver without conjugate gradients."""
     monkeypatch.setenv("GFNFF_EEQ_SOLVER", "batched")
     Z, X = workloads.alkane(64, 1001)
     g = GFNFF(precision=MIXED)
     assert g.setMolecule(Z, X), g.getErrorMessage()
-    assert g.eeqSolver() == "batched"
+    assert g.eeqSolver() == "batched" and g.batchKernel() == "tensor"
     e = g.calculateEnergy(True)
     assert not g.hasError(), g.getErrorMessage()
     T, Go, qo, cn = Oracle(Z, X).engrad(X)

@@ -22,7 +22,7 @@ def test_single_alkane(nc, monkeypatch):
     Z, X = workloads.alkane(nc, nc)
     g = GFNFF(precision=FP64)
     assert g.setMolecule(Z, X), g.getErrorMessage()
-    assert g.eeqSolver() == "batched"
+    assert g.eeqSolver() == "batched" and g.batchKernel() == "cg"
     rng = np.random.default_rng(nc)
     for step in range(3):   # the set-up geometry, then off it
         x = X + (0.03 * step) * rng.normal(size=X.shape).clip(-2, 2)
@@ -41,6 +41,7 @@ def test_batch_mixed_sizes_and_fragments():
     mols += [workloads.water_cluster(n, n) for n in (1, 7, 40)]
     g = GFNFF(precision=FP64)
     assert g.setMoleculeBatch(mols), g.getErrorMessage()
+    assert g.batchKernel() == "cg"
     for _ in range(3):   # repeated: no state of one evaluation reaches the next
         e, st = g.calculateEnergyBatch()
         assert (st == 0).all()
@@ -60,6 +61,7 @@ def test_batch_with_indefinite_molecule(monkeypatch):
             monkeypatch.setenv("GFNFF_BATCH_TC", "0")
         g = GFNFF(precision=FP64)
         assert g.setMoleculeBatch(mols), g.getErrorMessage()
+        assert g.batchKernel() == ("cholesky" if direct else "cg")
         out.append(g.calculateEnergyBatch())
     (e0, s0), (e1, s1) = out
     assert (s0 == s1).all()
