@@ -488,10 +488,17 @@ struct Engine::Impl {
     {
         cg_bins.clear();
         const size_t cap = 208 * 1024;
-        // a factorisation's time is that of its longest molecule until the chip is full, CG's grows
-        // with the number of CTAs from the start: 200 conformers (2.0 waves of CTAs) take 165 / 195
-        // us (mixed / FP64) against 255 / 510, 512 (5.1 waves) 393 / 453 against 306 / 666
-        const double waves = opt.precision == 1 ? 3.0 : 8.0;
+        // The time of a factorisation is that of its longest molecule until the chip is full, CG's grows with
+        // the number of CTAs from the start.  Conformers of 20 to 300 atoms, EEQ in us:
+        //   molecules (= 1/100 waves of CTAs)  100   200   300   400   512   700  1000  1500
+        //   mixed: CG                          140   184   255   295   424   506   725   983
+        //          tensor-core Cholesky        232   251   261   267   302   368   530   749
+        //   FP64:  CG                          147   191   262   319   446   514   781  1026
+        //          Cholesky                    493   507   524   533   671   782  1023  1308
+        // so the mixed form crosses at three waves and the FP64 form, at a steady 0.78, not at all.
+        int nsm = 0, smem_sm = 0;
+        CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, opt.device));
+        CK(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, opt.device));
         const int nm = (int)nr.size();
         std::vector<int> cs(nm, 1);
         int ctas = 0;
@@ -500,15 +507,15 @@ struct Engine::Impl {
             while (cs[m] < 8 && cg_smem(nr[m], na[m], cs[m]) > cap) cs[m] *= 2;
             if (cg_smem(nr[m], na[m], cs[m]) > cap) return;   // cg_on stays false
             ctas += cs[m];
-            slots += cs[m] > 1 ? cs[m] : std::max(1.0 / 8.0, cg_smem(nr[m], na[m], 1) / 222e3);
+            slots += cs[m] > 1 ? cs[m] : std::max(1.0 / 8.0, cg_smem(nr[m], na[m], 1) / (double)smem_sm);
         }
-        if (!any_size && slots > waves * 148.0) return;
+        if (!any_size && opt.precision == 1 && slots > 3.0 * nsm) return;
         // few molecules: larger clusters while the SMs hold one CTA each (a product and the
         // build shrink with the slice; below ~48 unknowns the barriers cost more)
         for (int top = 2; top <= 4; top *= 2) {
             int more = 0;
             for (int m = 0; m < nm; ++m) more += nr[m] > 24 * top && cs[m] < top ? top - cs[m] : 0;
-            if (ctas + more > 148) break;
+            if (ctas + more > nsm) break;
             for (int m = 0; m < nm; ++m)
                 if (nr[m] > 24 * top && cs[m] < top) cs[m] = top;
             ctas += more;
