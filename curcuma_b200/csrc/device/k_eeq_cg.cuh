@@ -227,6 +227,12 @@ __device__ __forceinline__ void cg_max(const double* v, const double* w, int n, 
     wmax = __uint_as_float(__reduce_max_sync(0xffffffffu, b));
 }
 
+// positive, and far from the ends of the range (2^-1007 .. 2^1007): a scalar that rcp_pos takes
+__device__ __forceinline__ bool cg_scalar(double v)
+{
+    return (unsigned)__double2hiint(v) - 0x01000000u < 0x7ee00000u - 0x01000000u;
+}
+
 // entry c of the start vector, in [-1, 1): the bits of c mixed by multiplications and shifts
 __device__ __forceinline__ double cg_start(int c)
 {
@@ -411,12 +417,12 @@ __global__ void __launch_bounds__(kCgThreads) k_eeq_cg(View V, CgArgs A)
         }
         const double beta = start ? 0.0 : rz * irz_old;
         const double pmp = start ? zw : zw - beta * rz * ialpha;
-        if (!(pmp > 0.0 && rz > 0.0)) {   // not positive definite, or not a number
+        if (!(cg_scalar(pmp) && cg_scalar(rz))) {   // not positive definite, or not a number
             state = 1;
             break;
         }
-        const double alpha = rz / pmp;
-        irz_old = 1.0 / rz;
+        const double alpha = rz * rcp_pos(pmp);   // a division is 0.25 us of dependent operations in every iteration
+        irz_old = rcp_pos(rz);
         ialpha = pmp * irz_old;
         __syncthreads();   // every warp has read r, z and w
         for (int q = threadIdx.x; q < nr; q += blockDim.x) {

@@ -23,8 +23,9 @@ def test_reciprocal_square_root(lo, hi):
     assert 0.0 <= u <= 2.0, u
 
 
-# (r^6 + r0^6)(r^8 + r0^8) of the D4 damping: r0 from 4.8 to some 20 bohr, r up to 50
-@pytest.mark.parametrize("lo,hi", [(1e9, 1e27), (1.0, 1e9)])
+# (r^6 + r0^6)(r^8 + r0^8) of the D4 damping: r0 from 4.8 to some 20 bohr, r up to 50; and the scalars of the
+# conjugate gradients, which are checked to lie within 2^-1007 .. 2^1007
+@pytest.mark.parametrize("lo,hi", [(1e9, 1e27), (1.0, 1e9), (1e-40, 1.0), (8e-304, 1e-40), (1e27, 1.3e303)])
 def test_reciprocal(lo, hi):
     u = _lib.load().gfnff_reciprocal_ulps(0, 0, lo, hi, N)
     assert 0.0 <= u <= 1.0, u
