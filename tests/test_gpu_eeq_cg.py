@@ -37,19 +37,28 @@ def test_single_alkane(nc, monkeypatch):
 
 
 def test_batch_mixed_sizes_and_fragments():
+    """At the set-up geometry, where the preconditioner is the matrix's own inverse, off it, and there again"""
     mols = [workloads.alkane(n, n) for n in (1, 2, 8, 30, 64, 100)]
     mols += [workloads.water_cluster(n, n) for n in (1, 7, 40)]
     g = GFNFF(precision=FP64)
     assert g.setMoleculeBatch(mols), g.getErrorMessage()
     assert g.batchKernel() == "cg"
-    for _ in range(3):   # repeated: no state of one evaluation reaches the next
+    rng = np.random.default_rng(4)
+    noise = [rng.normal(size=x.shape).clip(-2, 2) for _, x in mols]
+    iterations = []
+    for scale in (0.0, 0.02, 0.06, 0.0):   # no state of one evaluation reaches the next
+        xs = [x + scale * d for (_, x), d in zip(mols, noise)]
+        g.updateGeometry(np.concatenate(xs))
         e, st = g.calculateEnergyBatch()
         assert (st == 0).all()
-        Q = np.split(g.getCharges(), np.cumsum([len(z) for z, _ in mols])[:-1])
-        for (Z, X), em, qm in zip(mols, e, Q):
-            T, G, q, cn = Oracle(Z, X).engrad(X)
+        iterations.append(g.eeqIterations())
+        cuts = np.cumsum([len(z) for z, _ in mols])[:-1]
+        for (Z, X), x, em, qm, gm in zip(mols, xs, e, np.split(g.getCharges(), cuts), np.split(g.getGradient(), cuts)):
+            T, G, q, cn = Oracle(Z, X).engrad(x)
             assert abs(em - T["total"]) < 1e-9
             assert np.abs(qm - q).max() < 1e-10
+            assert np.abs(gm - G).max() < 1e-9
+    assert iterations[0] == iterations[3] < iterations[1] < iterations[2] < 30, iterations
 
 
 def test_batch_with_indefinite_molecule(monkeypatch):
