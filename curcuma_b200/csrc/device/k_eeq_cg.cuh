@@ -2,9 +2,10 @@
 // molecules of at most kStageAtoms atoms).  Included inside namespace gfnff by engine.cu.
 //
 // The reduced matrix M of a molecule changes little between geometries, so its inverse at the
-// set-up geometry (FP32, k_eeq_inv, once per set-up) is a preconditioner that needs 3-12 products
-// where a factorisation has nr dependent steps: k_eeq_batch's Cholesky takes 230 us for 193
-// unknowns, latency all of it.  Here the cluster's CTAs hold equal row slices of M (FP64, built
+// set-up geometry (FP32, k_eeq_inv, once per set-up) is a preconditioner that needs 4 products there,
+// 11-14 at 0.02 Angstrom of noise per coordinate, 14-19 at 0.06 and 16-27 at 0.12 (FP64 form, 26 to 302
+// atoms; 20 for a C8 chain bent by 2 rad), where a factorisation has nr dependent steps: k_eeq_batch's
+// Cholesky takes 230 us for 193 unknowns, latency all of it, and 27 products 108 us.  Here the cluster's CTAs hold equal row slices of M (FP64, built
 // from the atoms) and of the inverse (FP32, one bulk copy while M is built) in shared memory for
 // the whole solve; the vectors are replicated in every CTA, and a product's slice is stored into
 // all of them (DSMEM), so an iteration is two products from shared memory and two cluster
@@ -61,25 +62,21 @@ __host__ __device__ constexpr size_t cg_smem(int nr, int na, int cs)
 struct CgMol {
     double *x, *y, *z, *al, *ad, *br, *va;
     int *red, *anc;
-    int a0;   // first atom of the molecule
-    bool single, born, far;
+    bool single, born;
     double keps;
     __device__ double a(int i, int j) const
     {
         if (i == j) return ad[i];
         const double dx = x[i] - x[j], dy = y[i] - y[j], dz = z[i] - z[j];
         const double d2 = dx * dx + dy * dy + dz * dz, s = al[i] + al[j];
-        const double ir = rsqrt_pos(d2), r = d2 * ir;
+        // the square overflows above 1e154 bohr: 1/r = 0 (one comparison; a call to an out-of-line form, as in
+        // k_eeq_M_tiles, took 93 registers instead of 76, which the side streams' kernels miss)
+        const bool inf = __double2hiint(d2) == 0x7ff00000;
+        const double ir = inf ? 0.0 : rsqrt_pos(d2), r = inf ? d2 : d2 * ir;
         double v = ir;
         if (d2 < 36.0 * s) v = erf(r * rsqrt_pos(s)) * ir;
         if (born) v += born_p16(keps, r, br[i], br[j]);
         return v;
-    }
-    // `far` molecules: out of line, from the atoms in global memory
-    __device__ double m_far(const View& V, int r, int c) const
-    {
-        return eeq_far(V.pos, V.alpeeq, V.adiag, V.bdiag, V.brad, V.keps,
-                       make_int4(a0 + red[r], a0 + anc[r], a0 + red[c], a0 + anc[c]));
     }
     __device__ double m(int r, int c) const
     {
@@ -94,10 +91,8 @@ struct CgMol {
 __device__ void cg_stage(const View& V, const int* red2atom, const int* anchor, int r0, int nr, CgMol& S)
 {
     const int2 rg = V.jr[red2atom[r0]];
-    bool far = false;
     for (int i = threadIdx.x; i < rg.y - rg.x; i += blockDim.x) {
         const double4 p = V.pos[rg.x + i];
-        far |= far_coordinate(p.x, p.y, p.z);
         S.x[i] = p.x; S.y[i] = p.y; S.z[i] = p.z;
         S.al[i] = V.alpeeq[rg.x + i];
         S.ad[i] = V.adiag[rg.x + i] + (V.brad ? V.bdiag[rg.x + i] : 0.0);
@@ -111,8 +106,7 @@ __device__ void cg_stage(const View& V, const int* red2atom, const int* anchor, 
     S.single = anchor[red2atom[r0]] == anchor[red2atom[r0 + nr - 1]];
     S.born = V.brad != nullptr;
     S.keps = V.keps;
-    S.a0 = rg.x;
-    S.far = __syncthreads_or(far);
+    __syncthreads();
     if (S.single)
         for (int r = threadIdx.x; r < nr; r += blockDim.x) S.va[r] = S.a(S.red[r], S.anc[r]);
     __syncthreads();
@@ -336,15 +330,14 @@ __global__ void __launch_bounds__(kCgThreads) k_eeq_cg(View V, CgArgs A)
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
         // M u of the slice is stored into every CTA once all of them run
         if (CS > 1) asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-        auto build = [&](auto el) {
+        if (CS == 1) {   // each element once, into both triangles
+            for (int q = warp; q < rows; q += nw)
+                for (int c = lane; c <= q; c += 32) M[(size_t)q * nr + c] = M[(size_t)c * nr + q] = S.m(q, c);
+        } else {
             for (int q = warp; q < rows; q += nw) {
-                if (CS == 1) {   // each element once, into both triangles
-                    for (int c = lane; c <= q; c += 32) M[(size_t)q * nr + c] = M[(size_t)c * nr + q] = el(q, c);
-                    continue;
-                }
                 double g = 0.0;
                 for (int c = lane; c < nr; c += 32) {
-                    const double v = el(row0 + q, c);
+                    const double v = S.m(row0 + q, c);
                     M[(size_t)q * nr + c] = v;
                     g = fma(v, x[c], g);
                 }
@@ -352,9 +345,7 @@ __global__ void __launch_bounds__(kCgThreads) k_eeq_cg(View V, CgArgs A)
                 for (int o = 16; o > 0; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
                 if (lane < CS) cluster_store(w + row0 + q, lane, g);
             }
-        };
-        if (S.far) build([&](int r, int c) { return S.m_far(V, r, c); });
-        else build([&](int r, int c) { return S.m(r, c); });
+        }
     }
     for (int q = threadIdx.x; q < nr; q += blockDim.x) {
         const int k = A.red2atom[r0 + q];
