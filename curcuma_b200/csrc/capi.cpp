@@ -362,7 +362,7 @@ gfnff_status gfnff_energy_and_gradient_batch(gfnff_handle* h, const double* xyz,
         h->eng->enqueue(h->eng->d_xyz_scratch(), false);
         h->eng->fetch_batch(h->pin_terms.data(), h->pin_grad, st.data());
         // the CN neighbour list no longer covers this geometry: rebuild it around it (this
-        // evaluation used the all-pairs CN kernels)
+        // evaluation scanned the molecule)
         if (h->eng->cn_list_stale()) h->eng->refresh_cn_list();
     } catch (const std::exception& e) {
         return fail(h, GFNFF_CUDA_ERROR, e.what());
@@ -468,7 +468,7 @@ gfnff_status gfnff_energy_and_gradient(gfnff_handle* h, const double* xyz, doubl
             h->eng->fetch(h->pin_out, h->pin_grad, h->pin_status, nullptr);
         }
         // the CN neighbour list no longer covers this geometry: rebuild it around it (this
-        // evaluation used the all-pairs CN kernels)
+        // evaluation scanned the molecule)
         if (h->eng->cn_list_stale()) h->eng->refresh_cn_list();
     } catch (const std::exception& e) {
         return fail(h, GFNFF_CUDA_ERROR, e.what());

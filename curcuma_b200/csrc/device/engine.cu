@@ -1379,7 +1379,7 @@ void Engine::upload_batch(const std::vector<const Model*>& mols, const AlpbModel
     P.pos0.upload(p0); P.hbref.upload(p0); P.toporef.upload(p0); P.pos.alloc(n);
     {
         // the CN neighbour list is built from plain distances: a periodic cell takes the
-        // all-pairs CN kernels, which apply the minimum image to every pair
+        // scan of the molecule, which applies the minimum image to every pair
         const char* ecl = std::getenv("GFNFF_CN_LIST");
         P.cnl_on = !(ecl && !std::strcmp(ecl, "0")) && !P.cell.on;
         if (P.cnl_on) {

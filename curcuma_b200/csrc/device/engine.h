@@ -80,8 +80,8 @@ public:
     // same molecule with the same fragments, in place
     void update_eeq_parameters(const Model& m);
     // the CN neighbour list no longer covers the geometry of the last evaluation (its
-    // evaluations fell back to the all-pairs CN kernels); refresh_cn_list rebuilds it
-    // around that geometry
+    // evaluations scanned the molecule instead); refresh_cn_list rebuilds it around that
+    // geometry
     // (read_now: read the device flag; otherwise the value fetched with the last results)
     bool cn_list_stale(bool read_now = false);
     void refresh_cn_list();
@@ -92,8 +92,9 @@ public:
     // EEQ solver in use: "library", "tiled", "pcg", "lu" or "batched"
     const char* solver_name() const;
     // Coulomb + D4 pair kernel variant picked by the set-up autotuner: "sym32", "sym64",
-    // "sym64_occ10" or "rows"
+    // "sym64_occ10" (the largest tiles) or "rows"
     const char* pair_kernel_name() const;
+    // what solves the charges of a batch: "cg", "tensor" or "cholesky"
     const char* batch_kernel_name() const;
     // iterations of the last iterative EEQ solve (0 for direct solvers)
     int eeq_iterations();

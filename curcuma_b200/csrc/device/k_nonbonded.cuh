@@ -2,7 +2,9 @@
 // all-pairs Coulomb + D4 dispersion, self energy, CN chain rule and the outputs.
 // Included inside namespace gfnff by engine.cu (one translation unit).
 //
-// The all-pairs kernels share one layout: a block owns kTile consecutive atoms i (one per
+// The kernels that go over all pairs by rows (k_pairs, the plain form of the Coulomb and D4 pairs, and
+// k_resp_pairs) share one layout; the Coulomb and D4 pairs of the default path are in k_pairs.cuh, and CN,
+// repulsion and the chain rule take a warp per atom.  A block owns kTile consecutive atoms i (one per
 // thread) and walks the partners j of its molecule range in tiles of kTile staged through
 // shared memory, so every partner record is read from L2 once per block and broadcast to
 // all threads.  grid.y splits the partner range of an i-block (nsplit slices) so that small
@@ -147,8 +149,9 @@ __device__ __forceinline__ void cn_partners(const View& V, int i, const double4&
 }
 
 // NA: atoms per warp, one after the other for the CN and side by side (eight lanes each) for the
-// weights, whose logarithms and exponentials are the larger part of a large system's time (51,000
-// atoms: 58 us with one atom a warp); one where there are warps to spare.
+// weights, whose logarithms and exponentials are the larger part of a large system's time; one where
+// there are warps to spare.  Four against one, us: 3000 atoms 15.3 / 12.3, 5400 14.6 / 14.4, 8100 15.2 / 17.4,
+// 18,000 18.4 / 27.6; batches of 7700 atoms 17.3 / 17.2, 16,400 19.6 / 25.4, 52,600 36.6 / 61.9.
 template <class R, bool CELL, int NA>
 __global__ void __launch_bounds__(kBlock) k_cn_d4(View V, const int* __restrict__ off, const int* __restrict__ nbr,
                                                  const int* nl_bad)

@@ -14,18 +14,20 @@
 //    exchanges per 256 pairs, where one pair per lane needed 15-20 shuffles a pair;
 //  * 4 independent pairs per lane without a branch between them cover the latency of the FP64
 //    pipe; pairs within the width of the charges (erf, exp) are redone in one loop after them.
-// Measured on a B200, both kernels one after the other against one pair per lane and partner
-// tiles in shared memory: 20,480 atoms 2.42 -> 1.36 ms, 1000 waters 142 -> 72 us, 512 conformers
-// 285 -> 165 us, 194 atoms 70 -> 27 us.  Coulomb on 20,480 atoms: 0.56 ms, the FP64 pipe 50 % busy
-// (25 of 55 instructions a pair; 0.29 ms of FP64 issue); D4: 0.84 ms, latency of the operand loads
-// and the dependent chain (FP64 pipe 25 %).  One kernel for both terms was slower (1.38-2.0 ms):
+// Measured on a B200 with events, both kernels one after the other against one pair per lane and
+// partner tiles in shared memory: 20,480 atoms 2.42 -> 1.36 ms (largest tiles), 1000 waters 142 -> 72 us,
+// 512 conformers 285 -> 165 us, 194 atoms 70 -> 27 us (smallest tiles).  Under the profiler, which
+// starts every kernel cold, on 20,480 atoms: Coulomb (128 x 64) 0.57 ms, the FP64 pipe 49 % busy (25 of 55
+// instructions a pair; 0.29 ms of FP64 issue); D4 (32 x 64) 0.89 ms, latency of the operand loads and
+// the dependent chain (FP64 pipe 26 %).  One kernel for both terms was slower (1.38-2.0 ms, events):
 // the D4 part takes the registers of the Coulomb part, and far tiles cannot leave early.
 #pragma once
 
 namespace {
 
-// warps per SM the pair kernels are built for: 168 registers a thread without spills (16 warps
-// at 128 registers spilled and measured 3 % slower on the 20,480-atom cluster)
+// warps per SM the pair kernels are built for: 168 registers a thread, without spills but for the
+// exact-gradient form of Coulomb (FAR, 40-44 bytes); 16 warps at 128 registers spilled in every form and
+// measured 3 % slower on the 20,480-atom cluster
 constexpr int kPairWarps = 12;
 
 // c += A B, A 16 x 4 (lane: rows g and g + 8, column t), B 4 x 8 (lane: row t, column g),

@@ -232,11 +232,12 @@ gfnff_status gfnff_eeq_charges_noalloc(int natoms, int nfrag, const double* d_xy
 
 /* Name of the EEQ solver chosen for the handle's molecule at setup: "tiled" (the in-house
  * persistent tiled Cholesky), "pcg" (block-Jacobi conjugate gradients; FP64 true residual
- * <= 1e-12 max|b| in the FP64 form, <= 1e-10 in the mixed form), "batched" (per-molecule
- * conjugate gradients with the set-up inverse on a thread-block cluster, to the same FP64
- * residuals, with a direct elimination where they do not; a Cholesky for large batches), "lu" (indefinite matrix,
- * pivoted LU) or "library" (cuSOLVER's Cholesky, only when GFNFF_EEQ_SOLVER=library asks
- * for it); "" before setup.  The choice is made by timing the in-house solvers at setup.  curcuma's EEQSolver also picks among several solvers
+ * <= 1e-12 max|b| in the FP64 form, <= 1e-10 in the mixed form), "batched" (conjugate gradients
+ * with the set-up inverse on a thread-block cluster per molecule, to the same FP64 residuals, and a
+ * direct elimination where they do not converge; a Cholesky for large mixed batches), "lu"
+ * (indefinite matrix, pivoted LU) or "library" (cuSOLVER's Cholesky, only when
+ * GFNFF_EEQ_SOLVER=library asks for it); "" before setup.  The choice is made by timing the in-house
+ * solvers at setup.  curcuma's EEQSolver also picks among several solvers
  * (eeq_solver.cpp:1448-2086); this query has no counterpart there. */
 const char* gfnff_eeq_solver(gfnff_handle* h);
 

@@ -248,3 +248,41 @@ def test_fragments_whose_squared_distance_overflows(solver, monkeypatch):
         out.append((float(d_e[0]), d_g.cpu().numpy()))
     assert abs(out[0][0] - out[1][0]) < 1e-6    # 1 / (1e6 A) per pair of charges at most
     assert np.abs(out[0][1] - out[1][1]).max() < 1e-6
+
+
+@pytest.mark.parametrize("nc", [8, 30, 64])
+@pytest.mark.parametrize("angle", [0.5, 1.5])
+def test_chain_bent_far_from_its_setup(nc, angle, monkeypatch):
+    """One half of a chain turned about its middle: the set-up inverse is no longer that of the matrix, by
+    many Angstrom at the ends (device entry: no topology refresh).  Against the oracle at that geometry;
+    the products stay below those after which the solve is left to the elimination."""
+    import torch
+
+    monkeypatch.setenv("GFNFF_EEQ_SOLVER", "batched")
+    Z, X = workloads.alkane(nc, nc)
+    axis = int(np.argmax(np.ptp(X, axis=0)))
+    other = (axis + 1) % 3
+    c = X.mean(axis=0)
+    turn = np.eye(3)
+    turn[axis, axis] = turn[other, other] = np.cos(angle)
+    turn[other, axis], turn[axis, other] = np.sin(angle), -np.sin(angle)
+    x = X.copy()
+    half = X[:, axis] > c[axis]
+    x[half] = (X[half] - c) @ turn.T + c
+    g = GFNFF(precision=FP64)
+    assert g.setMolecule(Z, X), g.getErrorMessage()
+    d_x = torch.from_numpy(x / 0.529177210903).cuda()
+    d_e = torch.zeros(1, dtype=torch.float64, device="cuda")
+    d_g = torch.zeros(x.shape, dtype=torch.float64, device="cuda")
+    d_st = torch.full((1,), -1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert _lib.load().gfnff_energy_and_gradient_device(g.handle, d_x.data_ptr(), d_e.data_ptr(), d_g.data_ptr(),
+                                                        d_st.data_ptr()) == 0
+    torch.cuda.synchronize()
+    assert int(d_st[0]) == 0
+    T, G, q, cn = Oracle(Z, X).engrad(x)
+    scale = max(1.0, np.abs(G).max())   # atoms near the hinge come close
+    assert abs(float(d_e[0]) - T["total"]) < 1e-9 * max(1.0, abs(T["total"]))
+    assert np.abs(d_g.cpu().numpy() - G).max() < 1e-9 * scale
+    assert np.abs(g.getCharges() - q).max() < 1e-10
+    assert g.eeqIterations() < 20 + 2 * (len(Z) - 1) // 5, g.eeqIterations()
